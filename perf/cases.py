@@ -268,3 +268,134 @@ def tolerance(case):
         return {"rel": 1e-3, "max": 2.5e-3} if case["queries"] == 1 else {"rel": 2e-3, "max": 2e-2}
     deep = math.sqrt(case["layers"])
     return {"rel": 5e-3 * deep, "max": 2.5e-2 * deep, "differ": 0.01 if case["kv"] != "f16" else 0.0}
+
+
+# ------------------------------------------------------------------------------------------- the same in 64 bits
+
+
+def _block(w, nbytes):
+    """Packed rows as (N, super-blocks, bytes)."""
+    return w.reshape(w.shape[0], -1, nbytes)
+
+
+def _f16_at(blk, at):
+    return blk[..., at:at + 2].contiguous().view(torch.float16).double()
+
+
+def _weights64(fmt, w, scales=None):
+    """A packed matrix in 64 bits, (N, K)."""
+    if fmt == "q8_0":
+        return (w.double().view(w.shape[0], -1, 32) * scales.double().unsqueeze(-1)).view(w.shape)
+    if fmt == "q4_k":
+        blk = _block(w, 144)
+        s = blk[..., 4:16].int()
+        a, b, c = s[..., :4], s[..., 4:8], s[..., 8:]
+        scale = torch.cat([a & 63, (c & 15) | (a >> 6 << 4)], -1).double() * _f16_at(blk, 0)
+        least = torch.cat([b & 63, (c >> 4) | (b >> 6 << 4)], -1).double() * _f16_at(blk, 2)
+        qs = blk[..., 16:].unflatten(-1, (4, 32))
+        codes = torch.stack([qs & 15, qs >> 4], -2).flatten(-3, -2)
+        return (codes.double() * scale.unsqueeze(-1) - least.unsqueeze(-1)).flatten(1)
+    blk = _block(w, 210)
+    low = blk[..., :128].unflatten(-1, (2, 2, 32))
+    low = torch.cat([low & 15, low >> 4], -2)
+    high = blk[..., 128:192].unflatten(-1, (2, 1, 32))
+    high = torch.cat([(high >> s) & 3 for s in (0, 2, 4, 6)], -2)
+    codes = (low | high << 4).double() - 32
+    scale = blk[..., 192:208].contiguous().view(torch.int8).double() * _f16_at(blk, 208)
+    return (codes.flatten(-3).unflatten(-1, (16, 16)) * scale.unsqueeze(-1)).flatten(1)
+
+
+def _product64(x, w, fmt, scales=None):
+    """x W^T in 64 bits, some rows of W at a time."""
+    part = max(1, (1 << 27) // x.shape[-1])
+    return torch.cat([x @ _weights64(fmt, w[i:i + part], None if scales is None else scales[i:i + part]).T
+                      for i in range(0, w.shape[0], part)], -1)
+
+
+def _stored64(rows, kv):
+    """New K or V rows as a cache holds them: a q8_0 cache rounds them to its codes."""
+    if kv == "f16":
+        return rows
+    x = rows.half().float().unflatten(-1, (-1, 32))
+    s = (x.abs().amax(-1, keepdim=True) / 127).half().double()
+    return (torch.round(x.double() / s.clamp_min(1e-30)).clamp(-127, 127) * s).flatten(-2)
+
+
+def _cached64(kv, cache, i, n):
+    """The first n K and V rows of sequence i, (kv_heads, n, D) each."""
+    if kv == "f16":
+        return [c[i, :, :n].double() for c in cache]
+    if kv == "q8":
+        return [(cache[j][i, :, :n].double().unflatten(-1, (-1, 32)) * cache[j + 1][i, :, :n].double().unsqueeze(-1)).flatten(-2)
+                for j in (0, 2)]
+    table, pool = cache
+    pages = pool[table[i, :(n + 15) // 16].long()].unflatten(-1, (-1, 34))
+    rows = pages[..., 2:].contiguous().view(torch.int8).double() * _f16_at(pages, 0)
+    return [rows[:, j].flatten(-2).transpose(0, 1).flatten(1, 2)[:, :n] for j in (0, 1)]
+
+
+def _attention64(q, k, v, kv, cache, starts):
+    """Causal attention of new rows (batch, heads, tokens, D) over the cached ones before `starts` and themselves."""
+    out = []
+    for i, start in enumerate(starts):
+        ck, cv = (torch.cat([c, _stored64(new[i], kv)], 1) for c, new in zip(_cached64(kv, cache, i, start), (k, v)))
+        s, kv_h = q.shape[2], k.shape[1]
+        mask = torch.arange(start + s, device="cuda") > start + torch.arange(s, device="cuda").unsqueeze(1)
+        heads = []
+        for g in range(kv_h):
+            p = q[i].unflatten(0, (kv_h, -1))[g] @ ck[g].T / math.sqrt(D)
+            heads.append(p.masked_fill(mask, -math.inf).softmax(-1) @ cv[g])
+        out.append(torch.cat(heads))
+    return torch.stack(out)
+
+
+def _norm64(x, w, eps):
+    return x * (x.square().mean(-1, keepdim=True) + eps).rsqrt() * w.double()
+
+
+def _rope64(x, pos, inv_freq):
+    angle = (pos.float().unsqueeze(-1) * inv_freq).double().unsqueeze(1)        # (batch, 1, tokens, D / 2)
+    a, b = x.chunk(2, -1)
+    return torch.cat([a * angle.cos() - b * angle.sin(), b * angle.cos() + a * angle.sin()], -1)
+
+
+def _model64(c, dec, ids, pos):
+    """Logits of each sequence's last token; ids and pos are (batch, tokens)."""
+    s, (b, n) = dec.shape, ids.shape
+    x = _weights64("q4_k", dec.embed[ids.flatten()])
+    split = lambda t: t.view(b, n, -1, D).transpose(1, 2)
+    kv = "f16" if c["kv"] == "f16" else "paged"
+    for i, lw in enumerate(dec.layers):
+        y = _norm64(x, lw.norm_in, s.eps)
+        q, k, v = (split(_product64(y, w, fmt)) for w, fmt in ((lw.wq, "q4_k"), (lw.wk, "q4_k"), (lw.wv, "q6_k")))
+        q, k = _rope64(q, pos, dec.inv_freq), _rope64(k, pos, dec.inv_freq)
+        cache = (dec.k_cache[i], dec.v_cache[i]) if kv == "f16" else (dec.pools[i].page_table, dec.pools[i].pool)
+        a = _attention64(q, k, v, kv, cache, pos[:, 0].tolist())
+        x = x + _product64(a.transpose(1, 2).reshape(b * n, -1), lw.wo, "q4_k")
+        y = _norm64(x, lw.norm_post, s.eps)
+        y = torch.nn.functional.silu(_product64(y, lw.wg, "q4_k")) * _product64(y, lw.wu, "q4_k")
+        x = x + _product64(y, lw.wd, "q6_k")
+    return _product64(_norm64(x.view(b, n, -1)[:, -1], dec.norm_final, s.eps), dec.head, "q6_k")
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits; the caches hold copies and codes and have no such value."""
+    c, st = case, prepare(case, seed)
+    if c["kind"] == "linear":
+        x, w = st["x"].double(), st["w"]
+        if c["fmt"] == "q8_0":
+            y = [_product64(x, w[i], "q8_0", w[i + 1]) for i in range(0, len(w), 2)]
+        else:
+            y = [_product64(x, m, c["fmt"]) for m in w]
+        return torch.nn.functional.silu(y[0]) * y[1] if c["gated"] else y[0]
+    if c["kind"] == "attention":
+        starts = st["pos"].tolist() * (1 if c["kv"] == "paged" else c["batch"])
+        out = _attention64(*(st[n].double() for n in "qkv"), c["kv"], st["cache"], starts)
+        return (out,) + (None,) * len(st["cache"])
+    dec, b = st["dec"], c["batch"]
+    if c["kind"] == "prefill":
+        ids, first = st["ids"], torch.full((b, 1), c["start"], device="cuda")
+    else:
+        ids, first = dec.ids.view(b, 1), (dec.pos.expand(b) if c["kv"] == "f16" else dec.seq_pos).view(b, 1)
+    logits = _model64(c, dec, ids, first + torch.arange(ids.shape[1], device="cuda"))
+    return (logits,) + (None,) * (2 if c["kv"] == "f16" else 1)
