@@ -38,11 +38,17 @@
 #include <cuda.h>
 
 #include <climits>
+#include <type_traits>
 
 #include "linear.cuh"
 
 namespace alloyb {
 
+
+// Beyond this many tokens the residual is added by a kernel of its own after the GEMM: the GEMM's epilogue
+// holds one weight row per thread and fetches its residual values token by token (strided), which a single
+// tile per CTA hides and a walk over many tiles does not.
+constexpr int GEMM_FUSED_RESIDUAL_MAX_M = 128;
 
 namespace tc {
 
@@ -82,16 +88,20 @@ struct Cfg {
     // DG stages every group would wait for the MMAs of its own previous step before it may store the
     // next one; twice as many stages let it run a step ahead.
     static constexpr int STAGES = BM <= 128 ? 8 : 4;
-    static constexpr int DEC_WARPS = 4 * DG;
-    static constexpr int PACK_WARP = 2 + DEC_WARPS;             // warp 0 token copies, warp 1 MMA, then decode
-    static constexpr int EPI_WARP0 = PACK_WARP + 1;
+    // Warps 0-3: token copies, MMA, packed-row copies, (narrow tiles) a second MMA issuer; then the decode groups, then
+    // the epilogue, then further issuers.  Groups of four start at multiples of four: a warp's index modulo four is its
+    // quarter of tensor memory, and register counts are set by such groups.
+    static constexpr int PACK_WARP = 2, DEC_WARP0 = 4, EPI_WARP0 = DEC_WARP0 + 4 * DG;
+    // The 256-token tile runs 28 warps at 72 registers a thread: the epilogue, which holds 128 results per thread, takes
+    // over what the other roles can spare.  (56 x 128 + 56 x 512 + 112 x 256 = 72 x 896.)
+    static constexpr bool SHARE_REGS = BM == 256;
     // Under a narrow token tile an MMA is short and the issuing thread's own instruction stream (about a
-    // hundred cycles per tcgen05.mma) would pace the steps: NI threads (warp 1 and NI - 1 warps behind the
+    // hundred cycles per tcgen05.mma) would pace the steps: NI threads (warps 1 and 3, and two behind the
     // epilogue's) then issue a quarter or a half of every step's MMAs each, into an accumulator of their
     // own, and the epilogue adds the accumulators up.  (Worth 7 %: the decode warps bound these shapes.)
     static constexpr int NI = BM <= 32 ? 4 : (BM <= 64 ? 2 : 1);
-    static constexpr int MMA_WARP1 = EPI_WARP0 + EPI_THREADS / 32;      // issuers 1 .. NI-1
-    static constexpr int THREADS = (MMA_WARP1 + NI - 1) * 32;
+    static constexpr int MMA_WARP2 = EPI_WARP0 + EPI_THREADS / 32;      // issuers 2 and 3
+    static constexpr int THREADS = (MMA_WARP2 + (NI > 2 ? NI - 2 : 0)) * 32;
     // accumulators [gate/up][issuer] of BM columns each from column 0, decoded weights behind them
     static constexpr int W_COL0 = 2 * NI * BM <= 256 ? 2 * NI * BM : BM;
     static constexpr int TMEM_COLS = W_COL0 + STAGES * W_COLS <= 256 ? 256 : 512;
@@ -360,20 +370,24 @@ struct StageGate {
 
 // Decode k-step `ks` (0..3) of one Q4_K super-block of this thread's row: 64 weights = the low
 // nibbles (sub-block 2*ks, k 0..31 -> columns 0..15) and the high nibbles (sub-block 2*ks + 1,
-// k 32..63 -> columns 16..31) of 32 quant bytes.
-template <bool BF16>
-__device__ __forceinline__ void decode_q4k(const uint8_t* blk, int ks, uint32_t dst, StageGate& gate) {
-    const uint4 hdr = lds_u128(blk);
+// k 32..63 -> columns 16..31) of 32 quant bytes.  UPPER: ks >= 2 (sub-blocks 4-7, whose scales are put together from
+// two places) -- 0 or 1 where it is known at compile time, -1 where it is not.
+template <bool BF16, int UPPER>
+__device__ __forceinline__ void decode_q4k(const uint8_t* blk, const uint4& hdr, int ks, uint32_t dst, StageGate& gate) {
     const uint4 q0 = lds_u128(blk + 16 + ks * 32), q1 = lds_u128(blk + 32 + ks * 32);
     const float d = half_bits_to_f32(hdr.x & 0xffffu), dmin = half_bits_to_f32(hdr.x >> 16);
-    const uint64_t unbias = f2(-8388608.0f, -8388608.0f);
     const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    const uint64_t unbias = f2(-8388608.0f, -8388608.0f);
+    const bool upper = UPPER < 0 ? ks >= 2 : UPPER == 1;
+    const uint32_t sc4 = upper ? (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u) : hdr.y & 0x3f3f3f3fu;
+    const uint32_t mn4 = upper ? ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u) : hdr.z & 0x3f3f3f3fu;
+    const uint32_t sel = 0x7540u | (2u * (ks & 1));
 #pragma unroll
     for (int pl = 0; pl < 2; ++pl) {                     // nibble plane = sub-block 2*ks + pl
-        int sc, mn;
-        q4k_scale_min(hdr.y, hdr.z, hdr.w, 2 * ks + pl, sc, mn);
-        const float dl = d * static_cast<float>(sc), ml = dmin * static_cast<float>(mn);
-        const uint64_t dl2 = f2(dl, dl), ml2 = f2(-ml, -ml);
+        const float sc = __uint_as_float(__byte_perm(sc4, 0x4B000000u, sel + pl)) - 8388608.0f;
+        const float mn = __uint_as_float(__byte_perm(mn4, 0x4B000000u, sel + pl)) - 8388608.0f;
+        const float dl = d * sc, ml = -(dmin * mn);
+        const uint64_t dl2 = f2(dl, dl), ml2 = f2(ml, ml);
         uint32_t out[16];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -546,72 +560,10 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = bars->tmem_base;          // accumulator(s) from column 0; weight stages at W_COL0
     pdl_launch_dependents();
-    pdl_wait();
+    // Only the token copies and the epilogue touch what the previous kernel wrote (tokens, residual, outputs, split-K
+    // sums): they wait for it; packed rows are requested and decoded under its tail.
 
-    if (warp == 0) {
-        // ------------------------------------------------ token tiles
-        bool ok = true;
-        uint32_t it = 0;
-        for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-            const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
-            for (int sub = 0; sub < n_sub && ok; ++sub) {
-                for (int ks = im.sb0 * 4; ks < im.sb1 * 4 && ok; ++ks, ++it) {
-                    const uint32_t s = it % STAGES;
-                    if (it >= STAGES) ok = bar_wait(&bars->empty[s], ((it / STAGES) - 1) & 1);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    if (lane == 0) {
-                        bar_expect(&bars->full[s], X_STAGE);
-                        tma_2d(x_st + s * X_STAGE, &maps.x, ks * BK, im.tile_m * BM, &bars->full[s]);
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-    } else if (warp == C::PACK_WARP) {
-        // ------------------------------------------------ packed rows: one tensor copy per super-block
-        bool ok = true;
-        uint32_t sbi = 0;
-        for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
-            const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
-            for (int sub = 0; sub < n_sub && ok; ++sub) {
-                for (int sb = im.sb0; sb < im.sb1 && ok; ++sb, ++sbi) {
-                    const uint32_t ps = sbi % pstages;
-                    if (sbi >= static_cast<uint32_t>(pstages)) ok = bar_wait(&bars->p_empty[ps], ((sbi / pstages) - 1) & 1);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    if (lane == 0) {
-                        uint8_t* dst = p_st + ps * pstage_bytes;
-                        if (P.format == ALLOYB_Q4_K) {
-                            bar_expect(&bars->p_full[ps], Q4_STAGE);
-#pragma unroll
-                            for (int b = 0; b < PACK_BOXES; ++b)
-                                tma_2d(dst + b * PACK_BOX_ROWS * Q4_ROW, &maps.w[sub], sb * Q4K_BYTES, im.n0 + b * PACK_BOX_ROWS,
-                                       &bars->p_full[ps]);
-                        } else if (P.format == ALLOYB_Q6_K) {
-                            // a block is 2-byte aligned: copy the aligned window around it (reads past the
-                            // row's end are filled with zeros)
-                            bar_expect(&bars->p_full[ps], Q6_STAGE);
-#pragma unroll
-                            for (int b = 0; b < PACK_BOXES; ++b)
-                                tma_2d(dst + b * PACK_BOX_ROWS * Q6_ROW, &maps.w[sub], (sb * Q6K_BYTES) & ~15,
-                                       im.n0 + b * PACK_BOX_ROWS, &bars->p_full[ps]);
-                        } else {
-                            bar_expect(&bars->p_full[ps], Q8_STAGE);
-#pragma unroll
-                            for (int b = 0; b < PACK_BOXES; ++b) {
-                                const int r0 = b * PACK_BOX_ROWS;
-                                tma_2d(dst + r0 * 128, &maps.w[sub], sb * 256, im.n0 + r0, &bars->p_full[ps]);
-                                tma_2d(dst + Q8_HALF + r0 * 128, &maps.w[sub], sb * 256 + 128, im.n0 + r0, &bars->p_full[ps]);
-                                tma_2d(dst + 2 * Q8_HALF + r0 * 16, &maps.s[sub], sb * 16, im.n0 + r0, &bars->p_full[ps]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                }
-            }
-        }
-    } else if (warp == 1 || warp >= C::MMA_WARP1) {
+    auto issue_mma = [&](int issuer) {
         // ------------------------------------------------ MMA issue (one lane per issuer)
         // This ONE thread's instruction stream paces the tensor pipe (which queues about one instruction
         // behind the running one), so the loop is kept to a few dozen instructions per step: descriptors
@@ -624,7 +576,7 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
             const uint32_t d_lo = static_cast<uint32_t>(d0), d_hi = static_cast<uint32_t>(d0 >> 32);
             const uint32_t full0 = s32(&bars->full[0]), empty0 = s32(&bars->empty[0]), w_base = tmem + C::W_COL0;
             constexpr int NI = C::NI, KK = 4 / NI;              // this issuer's MMAs per step: kk0 .. kk0 + KK - 1
-            const int issuer = warp == 1 ? 0 : warp - C::MMA_WARP1 + 1, kk0 = issuer * KK;
+            const int kk0 = issuer * KK;
             bool ok = true;
             uint32_t it = 0, tl = 0;
             for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x, ++tl) {
@@ -657,61 +609,150 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
             }
         }
         __syncwarp();
-    } else if (warp < C::PACK_WARP) {
+    };
+
+    if (warp < C::DEC_WARP0) {
+        if (C::SHARE_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == 0) {
+            // ------------------------------------------------ token tiles
+            pdl_wait();
+            bool ok = true;
+            uint32_t it = 0;
+            for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
+                const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
+                for (int sub = 0; sub < n_sub && ok; ++sub) {
+                    for (int ks = im.sb0 * 4; ks < im.sb1 * 4 && ok; ++ks, ++it) {
+                        const uint32_t s = it % STAGES;
+                        if (it >= STAGES) ok = bar_wait(&bars->empty[s], ((it / STAGES) - 1) & 1);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        if (lane == 0) {
+                            bar_expect(&bars->full[s], X_STAGE);
+                            tma_2d(x_st + s * X_STAGE, &maps.x, ks * BK, im.tile_m * BM, &bars->full[s]);
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        } else if (warp == C::PACK_WARP) {
+            // ------------------------------------------------ packed rows: one tensor copy per super-block
+            bool ok = true;
+            uint32_t sbi = 0;
+            for (int w = blockIdx.x; w < n_items && ok; w += gridDim.x) {
+                const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
+                for (int sub = 0; sub < n_sub && ok; ++sub) {
+                    for (int sb = im.sb0; sb < im.sb1 && ok; ++sb, ++sbi) {
+                        const uint32_t ps = sbi % pstages;
+                        if (sbi >= static_cast<uint32_t>(pstages)) ok = bar_wait(&bars->p_empty[ps], ((sbi / pstages) - 1) & 1);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                        if (lane == 0) {
+                            uint8_t* dst = p_st + ps * pstage_bytes;
+                            if (P.format == ALLOYB_Q4_K) {
+                                bar_expect(&bars->p_full[ps], Q4_STAGE);
+#pragma unroll
+                                for (int b = 0; b < PACK_BOXES; ++b)
+                                    tma_2d(dst + b * PACK_BOX_ROWS * Q4_ROW, &maps.w[sub], sb * Q4K_BYTES, im.n0 + b * PACK_BOX_ROWS,
+                                           &bars->p_full[ps]);
+                            } else if (P.format == ALLOYB_Q6_K) {
+                                // a block is 2-byte aligned: copy the aligned window around it (reads past the
+                                // row's end are filled with zeros)
+                                bar_expect(&bars->p_full[ps], Q6_STAGE);
+#pragma unroll
+                                for (int b = 0; b < PACK_BOXES; ++b)
+                                    tma_2d(dst + b * PACK_BOX_ROWS * Q6_ROW, &maps.w[sub], (sb * Q6K_BYTES) & ~15,
+                                           im.n0 + b * PACK_BOX_ROWS, &bars->p_full[ps]);
+                            } else {
+                                bar_expect(&bars->p_full[ps], Q8_STAGE);
+#pragma unroll
+                                for (int b = 0; b < PACK_BOXES; ++b) {
+                                    const int r0 = b * PACK_BOX_ROWS;
+                                    tma_2d(dst + r0 * 128, &maps.w[sub], sb * 256, im.n0 + r0, &bars->p_full[ps]);
+                                    tma_2d(dst + Q8_HALF + r0 * 128, &maps.w[sub], sb * 256 + 128, im.n0 + r0, &bars->p_full[ps]);
+                                    tma_2d(dst + 2 * Q8_HALF + r0 * 16, &maps.s[sub], sb * 16, im.n0 + r0, &bars->p_full[ps]);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+            }
+        } else if (warp == 1 || C::NI > 1) {
+            issue_mma(warp == 1 ? 0 : 1);
+        }
+    } else if (warp < C::EPI_WARP0) {
+        if (C::SHARE_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         // ------------------------------------------------ decode: thread = weight row = the tensor-memory
         // lane this warp may access (its index modulo 4 picks the quarter); group g takes the k-steps whose
         // running count is g modulo DG
-        const int r = (warp & 3) * 32 + lane, g = (warp - 2) >> 2;
+        const int r = (warp & 3) * 32 + lane, g = (warp - C::DEC_WARP0) >> 2;
         const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::W_COL0;
-        bool ok = true;
-        uint32_t it = 0, sbi = 0;
-        for (int w = blockIdx.x; w < n_items; w += gridDim.x) {
-            const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
-            for (int sub = 0; sub < n_sub; ++sub) {
-                for (int sb = im.sb0; sb < im.sb1; ++sb, ++sbi) {
-                    const uint32_t ps = sbi % pstages;
-                    bool have = false;                   // this thread waited for the super-block's rows
-#pragma unroll 1
-                    for (int k4 = 0; k4 < 4; ++k4, ++it) {
-                        if (static_cast<int>(it % DG) != g) continue;
-                        const uint32_t s = it % STAGES;
-                        if (ok && !have) ok = bar_wait(&bars->p_full[ps], (sbi / pstages) & 1);
-                        have = true;
+        // A super-block is four k-steps and DG divides four: group g has the steps g, g + DG, ... of every super-block,
+        // so that a step's place in the block is known at compile time (DG = 2: up to the group's parity) and the header
+        // is read once.  Ring positions are counted, not divided out.  (Steps dealt out one by one, with divisions by the
+        // run-time ring depth, and two groups under the 256-token tile: 14336 x 4096 at 2048 tokens 237 us, now 216; gate/up
+        // at 32 tokens 56, now 50.)
+        auto decode_all = [&](auto format) {
+            constexpr int FMT = decltype(format)::value;
+            bool ok = true;
+            uint32_t sbi = 0, ps = 0, p_par = 0;
+            for (int w = blockIdx.x; w < n_items; w += gridDim.x) {
+                const Item im = item_of(w, tiles_n, tiles_m, nsb, P.splits);
+                for (int sb = n_sub * im.sb0; sb < n_sub * im.sb1; ++sb, ++sbi) {
+                    if (ok) ok = bar_wait(&bars->p_full[ps], p_par);
+                    const uint8_t* stg = p_st + ps * pstage_bytes;
+                    const uint8_t* row = FMT == ALLOYB_Q4_K ? stg + r * Q4_ROW : stg + r * Q6_ROW;
+                    uint4 hdr = make_uint4(0u, 0u, 0u, 0u);
+                    if (FMT == ALLOYB_Q4_K) hdr = lds_u128(row);
+                    // (a gate/up pair walks K twice: the block's place in its row starts over)
+                    const int k_sb = sb - im.sb0 * n_sub;
+                    const uint32_t off6 = ((im.sb0 + (k_sb >= im.sb1 - im.sb0 ? k_sb - (im.sb1 - im.sb0) : k_sb)) * Q6K_BYTES) & 15;
+                    auto step = [&](auto index) {
+                        constexpr int J = decltype(index)::value;
+                        const int ks = g + DG * J;
+                        const uint32_t it = sbi * 4 + ks, s = it % STAGES;
                         // the stage's previous use must be over before the first store to it, not before
                         // the loads and the arithmetic: test now, and only wait (inside the decode, right
                         // before its first tensor-memory store) if the test failed
                         const uint32_t e_bar = s32(&bars->empty[s]), e_par = ((it / STAGES) - 1) & 1;
                         const bool free_now = it < STAGES || bar_test_a(e_bar, e_par);
                         if (ok) {
-                            const uint8_t* stg = p_st + ps * pstage_bytes;
                             const uint32_t dst = lane_base + s * W_COLS;
                             StageGate gate{e_bar, e_par, free_now, true};
                             // rows past N arrive as zeros from the tensor copy and decode to zeros
-                            if (P.format == ALLOYB_Q4_K)
-                                decode_q4k<BF16>(stg + r * Q4_ROW, k4, dst, gate);
-                            else if (P.format == ALLOYB_Q6_K)
-                                decode_q6k<BF16>(stg + r * Q6_ROW + ((sb * Q6K_BYTES) & 15), k4, dst, gate);
-                            else
-                                decode_q8_0<BF16>(stg, k4, r, dst, gate);
+                            if (FMT == ALLOYB_Q4_K) decode_q4k<BF16, DG == 2 ? J : -1>(row, hdr, ks, dst, gate);
+                            else if (FMT == ALLOYB_Q6_K) decode_q6k<BF16>(row + off6, ks, dst, gate);
+                            else decode_q8_0<BF16>(stg, ks, r, dst, gate);
                             ok = gate.ok;
                             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         }
                         bar_arrive(&bars->full[s]);
-                    }
-                    // every decode thread releases the super-block once, after its last step of it (a
-                    // group with no step in it -- DG = 4 always has one -- releases it at once)
+                    };
+                    step(std::integral_constant<int, 0>{});
+                    if (DG == 2) step(std::integral_constant<int, DG == 2 ? 1 : 0>{});
+                    // every decode thread releases the super-block once, after its last step of it
                     bar_arrive(&bars->p_empty[ps]);
+                    if (++ps == static_cast<uint32_t>(pstages)) {
+                        ps = 0;
+                        p_par ^= 1;
+                    }
                 }
             }
-        }
-    } else {
+        };
+        static_assert(DG == 2 || DG == 4, "groups deal out the four steps of a super-block");
+        if (P.format == ALLOYB_Q4_K) decode_all(std::integral_constant<int, ALLOYB_Q4_K>{});
+        else if (P.format == ALLOYB_Q6_K) decode_all(std::integral_constant<int, ALLOYB_Q6_K>{});
+        else decode_all(std::integral_constant<int, ALLOYB_Q8_0>{});
+    } else if (C::NI <= 2 || warp < C::MMA_WARP2) {
+        if (C::SHARE_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         // ------------------------------------------------ epilogue: TMEM -> registers, release, -> C
         constexpr int HT = BM / 2;                          // tokens per thread
         const int ew = warp - C::EPI_WARP0;
         const int quarter = warp & 3;                       // TMEM lanes this warp may read
         const int half = ew >> 2;                           // token columns half*HT .. +HT-1
         const int et = threadIdx.x - C::EPI_WARP0 * 32;     // 0..255
+        pdl_wait();
         bool ok = true;
         uint32_t tl = 0;
         for (int w = blockIdx.x; w < n_items; w += gridDim.x, ++tl) {
@@ -721,14 +762,14 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
             if (ok) ok = bar_wait(&bars->acc_full, tl & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half * HT;
-            if (P.splits == 1) {
+            if (BM > SPLIT_MAX_BM || P.splits == 1) {
                 uint32_t acc[HT / 2];                       // this lane's row, two tokens per register
                 if (ok) {
 #pragma unroll
                     for (int c = 0; c < HT / 8; ++c) {
                         uint32_t v[8];
                         load_sum<C::NI, BM>(src + c * 8, v);
-                        if (P.gated) {
+                        if (BM <= SPLIT_MAX_BM && P.gated) {
                             uint32_t u[8];
                             load_sum<C::NI, BM>(src + C::NI * BM + c * 8, u);
 #pragma unroll
@@ -747,16 +788,18 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                     const int64_t ld = second ? P.ldy2 : P.ldy;
                     uint16_t* col = static_cast<uint16_t*>(second ? P.y2 : P.y) + static_cast<int64_t>(tok0) * ld +
                                     (second ? n - P.n_split : n);
-                    const uint16_t* res =
-                        P.residual ? static_cast<const uint16_t*>(P.residual) + static_cast<int64_t>(tok0) * P.ldy + n : nullptr;
+                    const uint16_t* res =           // (the 256-token tile's residual is added by a kernel of its own)
+                        BM <= GEMM_FUSED_RESIDUAL_MAX_M && P.residual ? static_cast<const uint16_t*>(P.residual) + static_cast<int64_t>(tok0) * P.ldy + n : nullptr;
+                    const int left = P.M - tok0;
 #pragma unroll
                     for (int e = 0; e < HT; ++e) {
-                        if (tok0 + e < P.M) {
+                        if (e < left) {
                             uint16_t o = static_cast<uint16_t>(e & 1 ? acc[e >> 1] >> 16 : acc[e >> 1] & 0xffffu);
                             // residual: dtype(residual + dtype(acc))
                             if (res) o = to_16<BF16>(to_f32<BF16>(res[static_cast<int64_t>(e) * P.ldy]) + to_f32<BF16>(o));
-                            col[static_cast<int64_t>(e) * ld] = o;
+                            *col = o;
                         }
+                        col += ld;
                     }
                 }
             } else {
@@ -836,6 +879,8 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                 asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");     // bars->last may be rewritten
             }
         }
+    } else {
+        issue_mma(warp - C::MMA_WARP2 + 2);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -912,7 +957,7 @@ static int launch(const Maps& maps, const Params& P, int grid, int dev, cudaStre
         if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
         configured[dev] = true;
     }
-    gemm_tc_kernel<BF16, BM, DG><<<grid, C::THREADS, C::SMEM_BYTES, st>>>(maps, P);
+    launch_pdl(gemm_tc_kernel<BF16, BM, DG>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, st, maps, P);
     return check_launch();
 }
 
@@ -922,7 +967,7 @@ static int launch_bm(int BM, const Maps& maps, const Params& P, int grid, int de
         case 32: return launch<BF16, 32, 4>(maps, P, grid, dev, st);
         case 64: return launch<BF16, 64, 4>(maps, P, grid, dev, st);
         case 128: return launch<BF16, 128, 4>(maps, P, grid, dev, st);
-        default: return launch<BF16, 256, 2>(maps, P, grid, dev, st);
+        default: return launch<BF16, 256, 4>(maps, P, grid, dev, st);
     }
 }
 
@@ -955,11 +1000,6 @@ __global__ void residual_add_kernel(uint16_t* __restrict__ y, const uint16_t* __
 }
 
 }  // namespace tc
-
-// Beyond this many tokens the residual is added by a kernel of its own after the GEMM: the GEMM's epilogue
-// holds one weight row per thread and fetches its residual values token by token (strided), which a single
-// tile per CTA hides and a walk over many tiles does not.
-constexpr int GEMM_FUSED_RESIDUAL_MAX_M = 128;
 
 int gemm_tc_residual_add(void* y, const void* residual, int M, int N, int64_t ldy, int dtype, cudaStream_t st) {
     const int64_t threads = static_cast<int64_t>(M) * ((N + 7) / 8);
