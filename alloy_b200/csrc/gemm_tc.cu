@@ -29,9 +29,8 @@
 // rows run ahead across item boundaries.  Eight epilogue warps drain the finished accumulator with
 // tcgen05.ld into REGISTERS, hand tensor memory back to the MMA warp at once, and only then store C (each
 // lane one weight row: a warp writes 64 contiguous bytes per token) while the next item's MMAs run.
-// When a matrix has fewer row tiles than the GPU has SMs and all tokens fit one tile, K is split: every
-// item adds its partial tile to a zeroed fp32 buffer (red.global) and the LAST item of a tile to finish
-// (a per-tile counter) reads the sums back, applies residual / activation, stores C and re-zeroes both.
+// When there are at most half as many tiles as SMs, K is split over a cluster of up to eight CTAs per tile: each leaves its
+// partial tile in its own shared memory and finishes a share of the tokens from all of them (distributed shared memory).
 // A gate/up pair runs as two K loops into two accumulators; the epilogue combines them.
 // Every wait is bounded: on a time-out the sticky device error word is set, the CTA still frees its
 // tensor memory and returns.
@@ -74,12 +73,8 @@ constexpr int PACK_BOXES = 4, PACK_BOX_ROWS = BN / PACK_BOXES;
 constexpr int DEC_GROUP = 128;          // one decode group: a thread per weight row
 constexpr int EPI_THREADS = 256;        // two per accumulator lane (half of the token columns each)
 constexpr uint32_t SPIN = 1u << 22;
-// Split-K scratch: fp32 sums [token][row] for up to SPLIT_MAX_ROWS rows (x 2 planes for a gate/up pair)
-// and SPLIT_MAX_BM tokens, and one counter per row tile.  Zero at load, re-zeroed by whoever finishes a
-// tile, so two GEMMs that split K must not overlap in time on one device.
-constexpr int SPLIT_MAX_TILES = 147, SPLIT_MAX_ROWS = SPLIT_MAX_TILES * BN, SPLIT_MAX_BM = 128;
-__device__ float g_split_sum[2 * SPLIT_MAX_BM * SPLIT_MAX_ROWS];
-__device__ unsigned int g_split_count[SPLIT_MAX_TILES];
+constexpr int GATED_MAX_BM = 128;       // tokens of a gate/up pair (two accumulators)
+constexpr int MAX_SPLITS = 8;           // K ranges of a tile = CTAs of a cluster
 
 template <int BM, int DG>
 struct Cfg {
@@ -105,6 +100,8 @@ struct Cfg {
     // accumulators [gate/up][issuer] of BM columns each from column 0, decoded weights behind them
     static constexpr int W_COL0 = 2 * NI * BM <= 256 ? 2 * NI * BM : BM;
     static constexpr int TMEM_COLS = W_COL0 + STAGES * W_COLS <= 256 ? 256 : 512;
+    // (split K: the token stages hold the fp32 partial tile(s) afterwards)
+    static_assert(STAGES * X_STAGE >= BM * BN * 4 * (BM <= GATED_MAX_BM ? 2 : 1), "partial tiles");
     static constexpr int SMEM_BYTES = 1024 /*align slack*/ + STAGES * X_STAGE + PACK_BYTES + 256;
     static_assert(W_COL0 + STAGES * W_COLS <= 512 && STAGES <= MAX_STAGES, "tensor memory");
 };
@@ -117,7 +114,6 @@ struct Bars {
     uint64_t acc_full;            // MMA -> epilogue (tcgen05.commit)
     uint64_t acc_empty;           // epilogue -> MMA (256 arrivals)
     uint32_t tmem_base;
-    uint32_t last;                // split-K: this CTA finished a tile last
 };
 static_assert(sizeof(Bars) <= 256, "barrier block");
 
@@ -480,10 +476,10 @@ struct Item {
 };
 __device__ __forceinline__ Item item_of(int w, int tiles_n, int tiles_m, int nsb, int splits) {
     Item it;
-    it.tile_n = w % tiles_n;
-    const int r = w / tiles_n, split = r / tiles_m;
+    const int split = w % splits, r = w / splits;
+    it.tile_n = r % tiles_n;
     it.n0 = it.tile_n * BN;
-    it.tile_m = r % tiles_m;
+    it.tile_m = r / tiles_n;
     it.sb0 = static_cast<int>(static_cast<int64_t>(split) * nsb / splits);
     it.sb1 = static_cast<int>(static_cast<int64_t>(split + 1) * nsb / splits);
     return it;
@@ -502,6 +498,23 @@ __device__ __forceinline__ float to_f32(uint16_t v) {
 template <bool BF16>
 __device__ __forceinline__ uint16_t to_16(float v) {
     return static_cast<uint16_t>(pack2<BF16>(v, 0.0f) & 0xffffu);
+}
+
+// All threads of the cluster: what was written to shared memory before is visible to the peers behind it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// v += the four floats at the same place in cluster rank k's shared memory.  (No memory clobber: several may be in
+// flight; volatile keeps them between the cluster barriers.)
+__device__ __forceinline__ void add_peer(float (&v)[4], const float* p, int k) {
+    uint32_t a;
+    float4 t;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(s32(p)), "r"(k));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(a));
+    v[0] += t.x;
+    v[1] += t.y;
+    v[2] += t.z;
+    v[3] += t.w;
 }
 
 // Eight columns of this thread's lane, summed over the NI issuers' accumulators (BM columns apart).
@@ -762,14 +775,14 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
             if (ok) ok = bar_wait(&bars->acc_full, tl & 1);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half * HT;
-            if (BM > SPLIT_MAX_BM || P.splits == 1) {
+            if (P.splits == 1) {
                 uint32_t acc[HT / 2];                       // this lane's row, two tokens per register
                 if (ok) {
 #pragma unroll
                     for (int c = 0; c < HT / 8; ++c) {
                         uint32_t v[8];
                         load_sum<C::NI, BM>(src + c * 8, v);
-                        if (BM <= SPLIT_MAX_BM && P.gated) {
+                        if (BM <= GATED_MAX_BM && P.gated) {
                             uint32_t u[8];
                             load_sum<C::NI, BM>(src + C::NI * BM + c * 8, u);
 #pragma unroll
@@ -803,10 +816,10 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                     }
                 }
             } else {
-                // split K: add this item's partial tile to the fp32 sums, [plane][token][row]
-                const int pitch = tiles_n * BN;
-                float* sum = g_split_sum + static_cast<int64_t>(tok0) * pitch + n;
-                const int64_t plane = static_cast<int64_t>(SPLIT_MAX_BM) * pitch;
+                // split K (a CTA has one item): leave the partial tile in shared memory -- the token stages are done with --
+                // as [plane][token][row] and finish this CTA's share of the tokens from the cluster's partial tiles, added
+                // in the order of the K ranges
+                float* sum = reinterpret_cast<float*>(x_st);
                 if (ok) {
                     for (int sub = 0; sub < n_sub; ++sub) {
 #pragma unroll
@@ -815,72 +828,58 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                             load_sum<C::NI, BM>(src + sub * C::NI * BM + c * 8, v);
 #pragma unroll
                             for (int e = 0; e < 8; ++e)
-                                if (tok0 + c * 8 + e < P.M)
-                                    atomicAdd(sum + sub * plane + static_cast<int64_t>(c * 8 + e) * pitch, __uint_as_float(v[e]));
+                                sum[(sub * BM + half * HT + c * 8 + e) * BN + quarter * 32 + lane] = __uint_as_float(v[e]);
                         }
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 }
                 bar_arrive(&bars->acc_empty);
-                // The last item of the tile to get here finishes it.  One release-acquire count per CTA: the
-                // barrier puts the epilogue threads' reductions before thread 0's release, the last CTA's acquire
-                // and its barrier put every item's reductions before the loads below.
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-                if (et == 0) {
-                    unsigned int old;
-                    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(&g_split_count[im.tile_n]) : "memory");
-                    bars->last = old == static_cast<unsigned int>(P.splits - 1) ? 1u : 0u;
-                    if (bars->last) g_split_count[im.tile_n] = 0u;
-                }
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");
-                if (bars->last && ok) {
-                    if (n < P.N) {
-                        const bool second = n >= P.n_split;
-                        const int64_t ld = second ? P.ldy2 : P.ldy;
-                        uint16_t* col = static_cast<uint16_t*>(second ? P.y2 : P.y) + static_cast<int64_t>(tok0) * ld +
-                                        (second ? n - P.n_split : n);
-                        const uint16_t* res = P.residual ? static_cast<const uint16_t*>(P.residual) +
-                                                               static_cast<int64_t>(tok0) * P.ldy + n
-                                                         : nullptr;
-                        // eight tokens' sums (and residuals) are requested together, then finished: one round
-                        // trip to L2 per eight tokens instead of one per token
-                        constexpr int FB = HT < 8 ? HT : 8;
-#pragma unroll 1
-                        for (int e0 = 0; e0 < HT; e0 += FB) {
-                            float v[FB], u[FB], r[FB];
+                cluster_sync();
+                const int rank = w % P.splits, t0 = rank * BM / P.splits, t1 = (rank + 1) * BM / P.splits;
+                const int r4 = (et & 31) * 4;                   // four rows per thread
+                // (four tokens' sums are requested together: a round trip to a peer per token would be the longest part)
+                constexpr int TB = 4, STEP = EPI_THREADS / 32;
+                for (int tb = t0 + (et >> 5); tb < t1 && im.tile_m * BM + tb < P.M; tb += TB * STEP) {
+                    float v[TB][4], u[TB][4];
 #pragma unroll
-                            for (int j = 0; j < FB; ++j) {
-                                const int e = e0 + j;
-                                const bool live = tok0 + e < P.M;
-                                const float* a = sum + static_cast<int64_t>(e) * pitch;
-                                v[j] = live ? __ldcg(a) : 0.f;
-                                u[j] = (live && P.gated) ? __ldcg(a + plane) : 0.f;
-                                r[j] = (live && res) ? to_f32<BF16>(res[static_cast<int64_t>(e) * P.ldy]) : 0.f;
+                    for (int q = 0; q < TB; ++q)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) v[q][e] = u[q][e] = 0.f;
+                    for (int k = 0; k < P.splits; ++k) {
+#pragma unroll
+                        for (int q = 0; q < TB; ++q)
+                            if (tb + q * STEP < t1) {
+                                add_peer(v[q], sum + (tb + q * STEP) * BN + r4, k);
+                                if (BM <= GATED_MAX_BM && P.gated) add_peer(u[q], sum + (BM + tb + q * STEP) * BN + r4, k);
                             }
+                    }
 #pragma unroll
-                            for (int j = 0; j < FB; ++j) {
-                                const int e = e0 + j;
-                                if (tok0 + e < P.M) {
-                                    float* a = sum + static_cast<int64_t>(e) * pitch;
-                                    __stcg(a, 0.0f);
-                                    float val = v[j];
-                                    if (P.gated) {
-                                        val = apply_act(val, P.act) * u[j];
-                                        __stcg(a + plane, 0.0f);
-                                    }
-                                    uint16_t o = to_16<BF16>(val);
-                                    if (res) o = to_16<BF16>(r[j] + to_f32<BF16>(o));
-                                    col[static_cast<int64_t>(e) * ld] = o;
-                                }
+                    for (int q = 0; q < TB; ++q) {
+                        const int tok = im.tile_m * BM + tb + q * STEP;
+                        if (tb + q * STEP >= t1 || tok >= P.M) continue;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int n1 = im.n0 + r4 + e;
+                            if (n1 < P.N) {
+                                const bool second = n1 >= P.n_split;
+                                const int64_t at = second ? static_cast<int64_t>(tok) * P.ldy2 + n1 - P.n_split : static_cast<int64_t>(tok) * P.ldy + n1;
+                                const float val = P.gated ? apply_act(v[q][e], P.act) * u[q][e] : v[q][e];
+                                uint16_t o = to_16<BF16>(val);
+                                if (P.residual) o = to_16<BF16>(to_f32<BF16>(static_cast<const uint16_t*>(P.residual)[at]) + to_f32<BF16>(o));
+                                static_cast<uint16_t*>(second ? P.y2 : P.y)[at] = o;
                             }
                         }
                     }
                 }
-                asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory");     // bars->last may be rewritten
+                cluster_sync();                                 // nobody's shared memory goes while a peer reads it
             }
         }
     } else {
         issue_mma(warp - C::MMA_WARP2 + 2);
+    }
+    if (P.splits > 1 && (warp < C::EPI_WARP0 || warp >= C::EPI_WARP0 + EPI_THREADS / 32)) {      // (the epilogue's are above)
+        cluster_sync();
+        cluster_sync();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -947,27 +946,58 @@ static int sm_count_of_device(int& dev) {
     return sms[dev];
 }
 
+// One CTA per SM walks the tiles (weight rows fastest, so neighbours share a token tile).  When the tiles are at most half
+// as many as the SMs, K is split over a cluster per tile: as many ranges as leave all clusters resident at once.  (The
+// partial tiles used to meet in a fixed fp32 scratch by atomic additions, for up to 128 tokens: two such GEMMs on
+// different streams added into each other's sums, and the order of the additions changed from run to run.)
 template <bool BF16, int BM, int DG>
-static int launch(const Maps& maps, const Params& P, int grid, int dev, cudaStream_t st) {
+static int launch(const Maps& maps, Params& P, int tiles, int sms, int dev, cudaStream_t st) {
     static bool configured[64] = {};
+    static int clusters[64][MAX_SPLITS + 1] = {};
     using C = Cfg<BM, DG>;
+    auto kern = gemm_tc_kernel<BF16, BM, DG>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(C::THREADS);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
     if (!configured[dev]) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(gemm_tc_kernel<BF16, BM, DG>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        for (int s = 2; s <= MAX_SPLITS && e == cudaSuccess; ++s) {
+            attr[0].val.clusterDim.x = s;
+            cfg.numAttrs = 1;
+            cfg.gridDim = dim3(s);
+            e = cudaOccupancyMaxActiveClusters(&clusters[dev][s], kern, &cfg);
+        }
         if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
         configured[dev] = true;
     }
-    launch_pdl(gemm_tc_kernel<BF16, BM, DG>, dim3(grid), dim3(C::THREADS), C::SMEM_BYTES, st, maps, P);
+    const int nsb = P.K / QK_K;
+    if (2 * tiles <= sms)
+        for (int s = 2; s <= MAX_SPLITS && s <= nsb; ++s)
+            if (tiles <= clusters[dev][s]) P.splits = s;
+    attr[0].val.clusterDim.x = P.splits;
+    cfg.numAttrs = 2;
+    const int items = tiles * P.splits;
+    cfg.gridDim = dim3(P.splits > 1 || items < sms ? items : sms);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, maps, P);
+    if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
     return check_launch();
 }
 
 template <bool BF16>
-static int launch_bm(int BM, const Maps& maps, const Params& P, int grid, int dev, cudaStream_t st) {
+static int launch_bm(int BM, const Maps& maps, Params& P, int tiles, int sms, int dev, cudaStream_t st) {
     switch (BM) {
-        case 32: return launch<BF16, 32, 4>(maps, P, grid, dev, st);
-        case 64: return launch<BF16, 64, 4>(maps, P, grid, dev, st);
-        case 128: return launch<BF16, 128, 4>(maps, P, grid, dev, st);
-        default: return launch<BF16, 256, 4>(maps, P, grid, dev, st);
+        case 32: return launch<BF16, 32, 4>(maps, P, tiles, sms, dev, st);
+        case 64: return launch<BF16, 64, 4>(maps, P, tiles, sms, dev, st);
+        case 128: return launch<BF16, 128, 4>(maps, P, tiles, sms, dev, st);
+        default: return launch<BF16, 256, 4>(maps, P, tiles, sms, dev, st);
     }
 }
 
@@ -1022,7 +1052,7 @@ int try_gemm_tc(const void* x, int M, int K, int dtype, const WeightSeg& seg, co
     if (dtype != ALLOYB_F16 && dtype != ALLOYB_BF16) return ALLOYB_NOT_TAKEN;
     if (seg.format != ALLOYB_Q4_K && seg.format != ALLOYB_Q6_K && seg.format != ALLOYB_Q8_0) return ALLOYB_NOT_TAKEN;
     if (M < GEMM_TC_MIN_M || K % QK_K) return ALLOYB_NOT_TAKEN;
-    if (up && M > SPLIT_MAX_BM) return ALLOYB_NOT_TAKEN;
+    if (up && M > GATED_MAX_BM) return ALLOYB_NOT_TAKEN;
     const bool q8 = seg.format == ALLOYB_Q8_0;
     if (q8 && (!seg.scales || reinterpret_cast<uintptr_t>(seg.scales) % 16 || seg.row_bytes != K)) return ALLOYB_NOT_TAKEN;
     if (q8 && up && (!up_scales || reinterpret_cast<uintptr_t>(up_scales) % 16)) return ALLOYB_NOT_TAKEN;
@@ -1041,14 +1071,7 @@ int try_gemm_tc(const void* x, int M, int K, int dtype, const WeightSeg& seg, co
     // that, and that seg.N is a whole number of row tiles); no residual, no gate/up pair, not Q8_0
     if (tail && (residual || up || q8 || seg.N % BN)) return ALLOYB_NOT_TAKEN;
     const int n_rows = seg.N + (tail ? tail->N : 0);
-    const int tiles_n = (n_rows + BN - 1) / BN, tiles_m = (M + BM - 1) / BM, nsb = K / QK_K;
-    // too few row tiles for the SMs and one token tile: split K (the sums live in a fixed scratch)
-    int splits = 1;
-    if (tiles_m == 1 && BM <= SPLIT_MAX_BM && tiles_n <= SPLIT_MAX_TILES && 2 * tiles_n <= sms) {
-        splits = sms / tiles_n;
-        if (splits > nsb) splits = nsb;
-    }
-
+    const int tiles_n = (n_rows + BN - 1) / BN, tiles_m = (M + BM - 1) / BM;
     Maps maps;
     bool ok = map2d(encode, &maps.x, dtype == ALLOYB_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
                     x, K, M, static_cast<uint64_t>(K) * 2, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B);
@@ -1083,14 +1106,12 @@ int try_gemm_tc(const void* x, int M, int K, int dtype, const WeightSeg& seg, co
     P.y2 = tail ? tail->y : nullptr;
     P.ldy2 = tail ? tail->ldy : 0;
     P.K = K;
-    P.splits = splits;
+    P.splits = 1;
     P.gated = up ? 1 : 0;
     P.act = act;
 
-    // persistent: one CTA per SM walks the items (weight-row tile fastest, so neighbours share a token tile)
-    const int n_items = tiles_n * tiles_m * splits;
-    const int grid = n_items < sms ? n_items : sms;
-    const int rc = dtype == ALLOYB_BF16 ? launch_bm<true>(BM, maps, P, grid, dev, st) : launch_bm<false>(BM, maps, P, grid, dev, st);
+    const int rc = dtype == ALLOYB_BF16 ? launch_bm<true>(BM, maps, P, tiles_n * tiles_m, sms, dev, st)
+                                        : launch_bm<false>(BM, maps, P, tiles_n * tiles_m, sms, dev, st);
     if (rc != ALLOYB_OK || !add_after) return rc;
     return gemm_tc_residual_add(seg.y, residual, M, seg.N, seg.ldy, dtype, st);
 }

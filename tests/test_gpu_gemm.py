@@ -201,3 +201,27 @@ def test_gemm_two_stacked_matrices_one_launch(fmt, m, nq, nk, k):
     for y, w in ((yq, wq), (yk, wk)):
         assert y.shape == (m, w.shape[0])
         assert_close(to_np(y), _ref(x, deq(w), torch.float16), torch.float16, f"stacked {fmt} m={m} rows={w.shape[0]}")
+
+
+@pytest.mark.parametrize("fmt,m,n,k,dt", [("q6_k", 333, 520, 2048, "f16"), ("q4_k", 150, 4096, 4096, "bf16"), ("q8_0", 600, 1000, 1024, "f16"),
+                                          ("q4_k", 40, 1152, 2304, "f16")])
+def test_gemm_split_over_a_cluster(fmt, m, n, k, dt):
+    """Few tiles, several token tiles among them: the K ranges of a tile meet in distributed shared memory.  The sums are
+    added in a fixed order and nothing is shared between launches: calls on two streams at once give the same bits."""
+    rng = np.random.default_rng([m, n, k])
+    tdt = DT[dt]
+    (wd, sd), w = _weights(fmt, rng, n, k)
+    x = torch.from_numpy(synth.activations(rng, m, k, np.float32)).to(tdt).to(DEV)
+    op = {"q4_k": lambda: torch.ops.alloy.gguf_q4_k_mm(x, wd), "q6_k": lambda: torch.ops.alloy.gguf_q6_k_mm(x, wd),
+          "q8_0": lambda: torch.ops.alloy.gguf_q8_0_mm(x, wd, sd)}[fmt]
+    y = op()
+    assert_close(to_np(y), _ref(x, w, tdt), tdt, f"cluster split {fmt} {m}x{n}x{k}")
+    torch.cuda.synchronize()
+    others = []
+    for _ in range(4):
+        for st in (torch.cuda.Stream(), torch.cuda.Stream()):
+            with torch.cuda.stream(st):
+                others.append(op())
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, o) for o in others)
+    assert _lib.load().alloyb_device_error(0) == 0
