@@ -67,3 +67,19 @@ def test_argmax_first_maximum(m, n, dt):
     xf = x.float()
     want = torch.tensor([int(torch.nonzero(xf[r] == xf[r].max())[0]) for r in range(m)])
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("b,h,kvh,d,dt", [(1, 32, 8, 128, torch.float16), (70, 5, 1, 64, torch.bfloat16), (3, 2, 2, 256, torch.float16),
+                                          (2, 3, 1, 48, torch.float16)])
+def test_rope_rows_equal_the_scalar_kernel(b, h, kvh, d, dt):
+    """Aligned 16-bit rows take the kernel that rotates eight pairs per thread, unaligned ones go element by element:
+    bit for bit the same."""
+    gen = torch.Generator().manual_seed(b)
+    q, k = torch.randn((b, h, d), generator=gen).to(dt).to(DEV), torch.randn((b, kvh, d), generator=gen).to(dt).to(DEV)
+    pos = torch.randint(0, 9000, (b,), generator=gen, dtype=torch.int32).to(DEV)
+    inv = (1.0 / (500000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d))).to(DEV)
+    q2 = torch.zeros(q.numel() + 1, dtype=dt, device=DEV)[1:].view(q.shape).copy_(q)
+    k2 = torch.zeros(k.numel() + 1, dtype=dt, device=DEV)[1:].view(k.shape).copy_(k)
+    ops.rope_inplace(q, k, pos, inv)
+    ops.rope_inplace(q2, k2, pos, inv)
+    assert torch.equal(q, q2) and torch.equal(k, k2)
