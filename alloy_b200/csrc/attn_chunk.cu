@@ -14,6 +14,12 @@
 // K/V tile in shared memory is shared by every row.  S = Q K^T and O += P V run on
 // mma.sync.m16n8k16 (fp16 operands, fp32 accumulation) with ldmatrix fragment loads; the softmax
 // is the usual online one in the exp2 frame; P enters the second product as fp16 hi + lo halves.
+//
+// What bounds it: a long prompt, the mma.sync pipe (three products of 64 x 64 x D per tile); a short chunk behind a long
+// history, the length of the chain of tiles.  So the next tile's K and V are copied (cp.async) while this one is computed
+// -- q8_0 caches: their raw bytes, which are expanded to the fp16 tile from shared memory --, and when the rows alone
+// give too few CTAs, the key range is split over a cluster of up to eight CTAs, which merge their partial results through
+// distributed shared memory (no scratch in global memory, one launch).
 #include "kv.cuh"
 
 namespace alloyb {
@@ -23,7 +29,8 @@ constexpr int ROWS = 64;          // (token, head) rows per CTA
 constexpr int KT = 64;            // KV tokens per tile
 constexpr int WARPS = 4;
 constexpr float NEG_BIG = -1.0e30f;
-constexpr float P_BIAS = 64.0f;   // keeps small probabilities out of fp16's subnormal range in the P * V product
+constexpr float NEG_LIVE = 0.5f * NEG_BIG;    // scores above it are real
+constexpr float P_BIAS_LOG2 = 6.0f;           // P * 64 keeps small probabilities out of fp16's subnormal range in the P * V product
 
 struct Params {
     const void* q;
@@ -37,6 +44,8 @@ struct Params {
     int G, Gp, HG;                // query heads per KV head; heads per CTA padded; CTAs per KV head
     float scale_log2;
     int* status;
+    int pool_aligned;             // paged: the pool starts on a 16-byte boundary
+    int splits;                   // CTAs (a cluster) that share the key range of the same rows
 };
 
 __device__ __forceinline__ uint32_t s32(const void* p) {
@@ -61,6 +70,22 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
+// A value of the same place in a cluster peer's shared memory.
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(s32(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ float peer_f32(const float* p, int rank) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(peer_addr(p, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 peer_f32x4(const float* p, int rank) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(peer_addr(p, rank)) : "memory");
+    return v;
+}
 __device__ __forceinline__ float q_as_f16(const void* q, int dtype, int64_t i) {
     // the attention runs on fp16 queries, like the reference (torch/ops/kv_quant.py:175-180)
     if (dtype == ALLOYB_F16) return __half2float(static_cast<const __half*>(q)[i]);
@@ -75,98 +100,157 @@ __device__ __forceinline__ void store_out(void* out, int dtype, int64_t i, float
     else *reinterpret_cast<float2*>(static_cast<float*>(out) + i) = make_float2(a, b);
 }
 
-// fp16(code * scale) of eight codes held in two 32-bit words -> four packed half2
-__device__ __forceinline__ uint4 dequant8(uint32_t w0, uint32_t w1, float scale) {
+// fp16(code * scale) of eight codes held in two 32-bit words -> four packed half2.  code + 128 becomes a half by one byte
+// permute (1024 + u), the subtraction is exact and the product of two halves is rounded once.
+__device__ __forceinline__ uint4 dequant8(uint32_t w0, uint32_t w1, __half2 scale) {
     uint32_t o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint32_t w = i < 2 ? w0 : w1;
-        const int c0 = static_cast<int8_t>((w >> (16 * (i & 1))) & 0xffu);
-        const int c1 = static_cast<int8_t>((w >> (16 * (i & 1) + 8)) & 0xffu);
-        o[i] = pack_h2(__fmul_rn(static_cast<float>(c0), scale), __fmul_rn(static_cast<float>(c1), scale));
+        const uint32_t u = (i < 2 ? w0 : w1) ^ 0x80808080u;
+        const uint32_t m = __byte_perm(u, 0x64646464u, (i & 1) ? 0x4342 : 0x4140);
+        const __half2 c = __hsub2(*reinterpret_cast<const __half2*>(&m), __float2half2_rn(1152.0f));
+        const __half2 v = __hmul2(c, scale);
+        o[i] = *reinterpret_cast<const uint32_t*>(&v);
     }
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// 16 bytes of global memory to shared memory, asynchronously; zeros when !live.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
 
-// Fill one 64-token tile of K (which = 0) or V (1) of (b, kvh) starting at token j0 into
-// dst[64][D + 8] as fp16; tokens >= n_kv become zero rows.
 template <int LAYOUT, int D>
-__device__ __forceinline__ void fill_tile(__half* dst, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
-    constexpr int PITCH = D + 8;
-    constexpr int NB = D / 32;
+struct Smem {
+    static constexpr int PITCH = D + 8;                                     // halves
+    static constexpr int TILE = KT * PITCH * 2;                             // an fp16 tile of K or V
+    static constexpr bool RAW = LAYOUT != ALLOYB_KV_F16;
+    static constexpr int RAW_ROW = LAYOUT == ALLOYB_KV_Q8_PAGED ? D / 32 * KV_BLOCK_BYTES : D;
+    static constexpr int RAW_TILE = KT * RAW_ROW;
+    static constexpr int Q = ROWS * PITCH * 2;
+    static constexpr int TILES = RAW ? 2 * TILE + 4 * RAW_TILE : 4 * TILE;  // fp16: two stages; q8: one tile, two raw stages
+    static constexpr int BYTES = Q + (TILES > ROWS * D * 4 ? TILES : ROWS * D * 4) + 2 * ROWS * 4;
+};
+
+// Request tile j0 (64 tokens) of K (which = 0) or V (1): fp16 rows into the tile itself, q8 bytes into the raw buffer.
+template <int LAYOUT, int D>
+__device__ __forceinline__ void request_tile(uint32_t dst, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
+    using M = Smem<LAYOUT, D>;
     const int tid = threadIdx.x;
-    if (LAYOUT == ALLOYB_KV_F16) {
-        const __half* base = static_cast<const __half*>(which ? P.kv.v0 : P.kv.k0) +
-                             (static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max * D;
-        for (int i = tid; i < KT * (D / 8); i += WARPS * 32) {
-            const int tok = i / (D / 8), c = i - tok * (D / 8);
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (j0 + tok < n_kv) v = __ldg(reinterpret_cast<const uint4*>(base + static_cast<int64_t>(j0 + tok) * D) + c);
-            *reinterpret_cast<uint4*>(dst + tok * PITCH + c * 8) = v;
-        }
-    } else if (LAYOUT == ALLOYB_KV_Q8_SPLIT) {
-        const int64_t row0 = (static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max;
-        const int8_t* codes = static_cast<const int8_t*>(which ? P.kv.v0 : P.kv.k0);
-        const __half* scales = static_cast<const __half*>(which ? P.kv.v1 : P.kv.k1);
-        // one thread per (token, 16 codes)
-        for (int i = tid; i < KT * (D / 16); i += WARPS * 32) {
-            const int tok = i / (D / 16), c = i - tok * (D / 16);
-            uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-            if (j0 + tok < n_kv) {
-                const int64_t row = row0 + j0 + tok;
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(codes + row * D) + c);
-                const float s = __half2float(__ldg(scales + row * NB + c / 2));
-                lo = dequant8(w.x, w.y, s);
-                hi = dequant8(w.z, w.w, s);
-            }
-            *reinterpret_cast<uint4*>(dst + tok * PITCH + c * 16) = lo;
-            *reinterpret_cast<uint4*>(dst + tok * PITCH + c * 16 + 8) = hi;
-        }
-    } else {
+    if (LAYOUT == ALLOYB_KV_Q8_PAGED) {
+        // whole pages: a head's slab of 16 rows is contiguous
+        constexpr int SLAB16 = PAGE_TOKENS * M::RAW_ROW / 16;
         const int32_t* table = static_cast<const int32_t*>(P.kv.k1) + static_cast<int64_t>(b) * P.kv.max_pages;
         const uint8_t* pool = static_cast<const uint8_t*>(P.kv.k0);
-        // one thread per (token, 32-code block); blocks are 2-byte aligned: 16-bit loads
-        for (int i = tid; i < KT * NB; i += WARPS * 32) {
-            const int tok = i / NB, blk = i - tok * NB;
-            uint4 o[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) o[u] = make_uint4(0u, 0u, 0u, 0u);
-            const int j = j0 + tok;
-            if (j < n_kv) {
-                const int64_t page = table[j / PAGE_TOKENS];
-                if (page < 0 || page >= P.kv.num_pages) {
-                    if (P.status) atomicOr(P.status, KV_STATUS_PAGE_RANGE);
-                } else {
-                    const uint16_t* bp = reinterpret_cast<const uint16_t*>(
-                        pool + paged_row_offset(page, which, kvh, j % PAGE_TOKENS, P.KV_H, D) + blk * KV_BLOCK_BYTES);
-                    const float s = half_bits_to_f32(__ldg(bp));
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const uint32_t a0 = __ldg(bp + 1 + 4 * u), a1 = __ldg(bp + 2 + 4 * u);
-                        const uint32_t a2 = __ldg(bp + 3 + 4 * u), a3 = __ldg(bp + 4 + 4 * u);
-                        o[u] = dequant8(a0 | (a1 << 16), a2 | (a3 << 16), s);
-                    }
+        for (int pg = 0; pg < KT / PAGE_TOKENS; ++pg) {
+            const int j = j0 + pg * PAGE_TOKENS;
+            const int64_t page = j < n_kv ? table[j / PAGE_TOKENS] : -1;
+            const bool live = page >= 0 && page < P.kv.num_pages;
+            if (j < n_kv && !live && tid == 0 && P.status) atomicOr(P.status, KV_STATUS_PAGE_RANGE);
+            const uint8_t* src = pool + (live ? paged_row_offset(page, which, kvh, 0, P.KV_H, D) : 0);
+            for (int i = tid; i < SLAB16; i += WARPS * 32) {
+                if (P.pool_aligned) {
+                    copy16(dst + (pg * SLAB16 + i) * 16, src + i * 16, live);
+                } else {                                 // a pool that starts off a 16-byte boundary (it is 2-byte aligned)
+                    const uint16_t* h = reinterpret_cast<const uint16_t*>(src + i * 16);
+#pragma unroll 1
+                    for (int e = 0; e < 8; ++e)
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + (pg * SLAB16 + i) * 16 + 2 * e), "h"(live ? __ldg(h + e) : uint16_t(0)) : "memory");
                 }
             }
+        }
+    } else {
+        constexpr int PER = (LAYOUT == ALLOYB_KV_F16 ? D * 2 : D) / 16, PITCH_B = LAYOUT == ALLOYB_KV_F16 ? M::PITCH * 2 : D;
+        const uint8_t* base = static_cast<const uint8_t*>(which ? P.kv.v0 : P.kv.k0) + (static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max * (PER * 16);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) *reinterpret_cast<uint4*>(dst + tok * PITCH + blk * 32 + u * 8) = o[u];
+        for (int i = tid; i < KT * PER; i += WARPS * 32) {
+            const int tok = i / PER, c = i - tok * PER;
+            const bool live = j0 + tok < n_kv;
+            copy16(dst + tok * PITCH_B + c * 16, base + static_cast<int64_t>(live ? j0 + tok : 0) * (PER * 16) + c * 16, live);
+        }
+    }
+}
+
+// The split layout's scales of this thread's blocks (see expand_tile), loaded a tile ahead.
+template <int D>
+struct Scales {
+    __half s[D / 64];
+};
+template <int LAYOUT, int D>
+__device__ __forceinline__ void load_scales(Scales<D>& o, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
+    if (LAYOUT != ALLOYB_KV_Q8_SPLIT) return;
+    constexpr int NB = D / 32;
+    const int tok = threadIdx.x >> 1, j = min(j0 + tok, n_kv - 1);
+    const __half* src = static_cast<const __half*>(which ? P.kv.v1 : P.kv.k1) +
+                        ((static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max + j) * NB + (threadIdx.x & 1) * (NB / 2);
+#pragma unroll
+    for (int i = 0; i < NB / 2; ++i) o.s[i] = __ldg(src + i);
+}
+
+// Raw q8_0 bytes of a tile -> fp16(code * scale): two threads per token, half of its 32-code blocks each; tokens at or past
+// n_kv become zero rows (whatever their page holds).
+template <int LAYOUT, int D>
+__device__ __forceinline__ void expand_tile(__half* dst, uint32_t raw, const Scales<D>& sc, int j0, int n_kv) {
+    using M = Smem<LAYOUT, D>;
+    constexpr int NB = D / 32;
+    const int tok = threadIdx.x >> 1, b0 = (threadIdx.x & 1) * (NB / 2);
+    const bool live = j0 + tok < n_kv;
+#pragma unroll
+    for (int i = 0; i < NB / 2; ++i) {
+        uint32_t w[8];
+        __half s;
+        if (LAYOUT == ALLOYB_KV_Q8_PAGED) {
+            const uint32_t at = raw + tok * M::RAW_ROW + (b0 + i) * KV_BLOCK_BYTES, base = at & ~3u, sh = (at & 2u) * 8u;
+            // scale, then 32 codes: nine words from the word that holds the scale, shifted into place
+            uint32_t x[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) x[k] = lds32(base + 4 * k);
+            s = __ushort_as_half(static_cast<unsigned short>(sh ? x[0] >> 16 : x[0] & 0xffffu));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = sh ? x[k + 1] : __funnelshift_r(x[k], x[k + 1], 16);
+        } else {
+            const uint32_t at = raw + tok * M::RAW_ROW + (b0 + i) * 32;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) w[k] = lds32(at + 4 * k);
+            s = sc.s[i];
+        }
+        const __half2 s2 = __half2half2(s);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            uint4 o = dequant8(w[2 * u], w[2 * u + 1], s2);
+            if (!live) o = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(dst + tok * M::PITCH + (b0 + i) * 32 + u * 8) = o;
         }
     }
 }
 
 template <int LAYOUT, int D>
 __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) {
+    using M = Smem<LAYOUT, D>;
     pdl_launch_dependents();
-    constexpr int PITCH = D + 8;
+    constexpr int PITCH = M::PITCH;
     extern __shared__ __align__(16) uint8_t smem[];
     __half* Qs = reinterpret_cast<__half*>(smem);
-    __half* Ks = Qs + ROWS * PITCH;
-    __half* Vs = Ks + KT * PITCH;
+    uint8_t* tiles = smem + M::Q;
+    float* Ms = reinterpret_cast<float*>(smem + M::BYTES - 2 * ROWS * 4);   // merge: row maxima, row sums
+    float* Ls = Ms + ROWS;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int split = blockIdx.x % P.splits;                // rank in the cluster
     const int kvh = blockIdx.y / P.HG, hgrp = blockIdx.y - kvh * P.HG, b = blockIdx.z;
     const int TQ = ROWS / P.Gp;                         // query tokens per CTA
-    const int tok0 = blockIdx.x * TQ;
+    // the last rows, which see the most keys, go first
+    const int tok0 = (gridDim.x / P.splits - 1 - blockIdx.x / P.splits) * TQ;
     const int gp_shift = P.Gp == 1 ? 0 : (P.Gp == 2 ? 1 : (P.Gp == 4 ? 2 : 3));
     const int heads_here = min(8, P.G - hgrp * 8);      // live heads of this CTA
     pdl_wait();
@@ -177,19 +261,42 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
     }
     const int tok_last = min(P.S, tok0 + TQ) - 1;
     const int n_kv = start + tok_last + 1;              // positions this CTA may read
+    const int n_tiles = (n_kv + KT - 1) / KT, per = (n_tiles + P.splits - 1) / P.splits;
+    const int tile0 = split * per, tile1 = min(n_tiles, tile0 + per);
+
+    auto request = [&](int tile, int buf) {
+        const uint32_t at = s32(tiles) + (M::RAW ? 2 * M::TILE + buf * 2 * M::RAW_TILE : buf * 2 * M::TILE);
+        request_tile<LAYOUT, D>(at, P, 0, b, kvh, tile * KT, n_kv);
+        request_tile<LAYOUT, D>(at + (M::RAW ? M::RAW_TILE : M::TILE), P, 1, b, kvh, tile * KT, n_kv);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    Scales<D> sk, sv;
+    if (tile0 < tile1) {
+        request(tile0, 0);
+        load_scales<LAYOUT, D>(sk, P, 0, b, kvh, tile0 * KT, n_kv);
+        load_scales<LAYOUT, D>(sv, P, 1, b, kvh, tile0 * KT, n_kv);
+    }
 
     // ---- Q rows -> shared memory (fp16); dead rows are zero
-    for (int i = threadIdx.x; i < ROWS * (D / 2); i += WARPS * 32) {
-        const int r = i / (D / 2), d = (i - r * (D / 2)) * 2;
+    const bool q_vec = P.q_dtype == ALLOYB_F16 &&
+                       ((reinterpret_cast<uintptr_t>(P.q) | (P.q_bs * 2) | (P.q_hs * 2) | (P.q_ts * 2)) & 15) == 0;
+    for (int i = threadIdx.x; i < ROWS * (D / 8); i += WARPS * 32) {
+        const int r = i / (D / 8), d = (i - r * (D / 8)) * 8;
         const int tl = r >> gp_shift, hg = r & (P.Gp - 1);
-        float a = 0.f, c = 0.f;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (tok0 + tl < P.S && hg < heads_here) {
             const int64_t base = b * P.q_bs + static_cast<int64_t>(kvh * P.G + hgrp * 8 + hg) * P.q_hs +
                                  static_cast<int64_t>(tok0 + tl) * P.q_ts + d;
-            a = q_as_f16(P.q, P.q_dtype, base);
-            c = q_as_f16(P.q, P.q_dtype, base + 1);
+            if (q_vec) {
+                v = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(P.q) + base));
+            } else {
+                uint32_t* e = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    e[k] = pack_h2(q_as_f16(P.q, P.q_dtype, base + 2 * k), q_as_f16(P.q, P.q_dtype, base + 2 * k + 1));
+            }
         }
-        *reinterpret_cast<uint32_t*>(Qs + r * PITCH + d) = pack_h2(a, c);
+        *reinterpret_cast<uint4*>(Qs + r * PITCH + d) = v;
     }
 
     // this thread's two rows: warp*16 + g and + 8
@@ -202,21 +309,40 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
         row_live[rr] = tok0 + tl < P.S && hg < heads_here;
         row_pos[rr] = start + tok0 + tl;
     }
+    const int first_pos = start + tok0 + ((warp * 16) >> gp_shift);      // the warp's earliest row
 
     float o[D / 8][4];
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m_run[2] = {NEG_BIG, NEG_BIG}, l_run[2] = {0.f, 0.f};
+    float m_run[2] = {NEG_BIG, NEG_BIG}, l_run[2] = {0.f, 0.f};          // (l times 64, like o)
 
     const uint32_t q_addr = s32(Qs + (warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + ((lane >> 4) & 1) * 8);
-    const uint32_t k_addr = s32(Ks + ((lane & 7) + ((lane >> 4) & 1) * 8) * PITCH + ((lane >> 3) & 1) * 8);
-    const uint32_t v_addr = s32(Vs + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + ((lane >> 4) & 1) * 8);
+    const uint32_t k_off = (((lane & 7) + ((lane >> 4) & 1) * 8) * PITCH + ((lane >> 3) & 1) * 8) * 2;
+    const uint32_t v_off = (((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + ((lane >> 4) & 1) * 8) * 2;
 
-    for (int j0 = 0; j0 < n_kv; j0 += KT) {
-        __syncthreads();                                // previous tile fully consumed (and Q stored)
-        fill_tile<LAYOUT, D>(Ks, P, 0, b, kvh, j0, n_kv);
-        fill_tile<LAYOUT, D>(Vs, P, 1, b, kvh, j0, n_kv);
-        __syncthreads();
+    for (int tile = tile0; tile < tile1; ++tile) {
+        const int buf = (tile - tile0) & 1, j0 = tile * KT;
+        const bool more = tile + 1 < tile1;
+        if (more) {
+            request(tile + 1, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();                                // this tile has arrived for every thread (and Q is stored)
+        uint32_t k_tile = s32(tiles) + buf * 2 * M::TILE;
+        if (M::RAW) {
+            const uint32_t raw = s32(tiles) + 2 * M::TILE + buf * 2 * M::RAW_TILE;
+            expand_tile<LAYOUT, D>(reinterpret_cast<__half*>(tiles), raw, sk, j0, n_kv);
+            expand_tile<LAYOUT, D>(reinterpret_cast<__half*>(tiles + M::TILE), raw + M::RAW_TILE, sv, j0, n_kv);
+            if (more) {
+                load_scales<LAYOUT, D>(sk, P, 0, b, kvh, j0 + KT, n_kv);
+                load_scales<LAYOUT, D>(sv, P, 1, b, kvh, j0 + KT, n_kv);
+            }
+            k_tile = s32(tiles);
+            __syncthreads();
+        }
+        const uint32_t k_addr = k_tile + k_off, v_addr = k_tile + M::TILE + v_off;
 
         // ---- S = Q K^T : 16 rows x 64 tokens per warp
         float s[KT / 8][4];
@@ -234,33 +360,41 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
                 mma16816(s[2 * n2 + 1], a, bq[2], bq[3]);
             }
         }
-        // ---- mask + online softmax (rows g and g + 8; columns 8n + 2t, + 1)
+        // ---- mask (tiles that reach past the warp's earliest row only) + online softmax (rows g and g + 8; columns
+        // 8n + 2t, + 1)
+        if (j0 + KT - 1 > first_pos) {
+#pragma unroll
+            for (int n = 0; n < KT / 8; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (j0 + 8 * n + 2 * t + (e & 1) > row_pos[e >> 1]) s[n][e] = NEG_BIG;
+        }
         float mx[2] = {NEG_BIG, NEG_BIG};
 #pragma unroll
         for (int n = 0; n < KT / 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int rr = e >> 1;
-                const int j = j0 + 8 * n + 2 * t + (e & 1);
-                const float v = (j <= row_pos[rr]) ? s[n][e] * P.scale_log2 : NEG_BIG;
-                s[n][e] = v;
-                mx[rr] = fmaxf(mx[rr], v);
+                // (a score of -inf or below the masked value counts as masked, NaN as absent, as it is below)
+                mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
             }
-        float alpha[2];
+        float alpha[2], m_sub[2];
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 1));
             mx[rr] = fmaxf(mx[rr], __shfl_xor_sync(0xffffffffu, mx[rr], 2));
-            const float m_new = fmaxf(m_run[rr], mx[rr]);
-            alpha[rr] = exp2f(m_run[rr] - m_new);
+            const float m_new = fmaxf(m_run[rr], mx[rr] > NEG_LIVE ? mx[rr] * P.scale_log2 : NEG_BIG);
+            alpha[rr] = ex2(m_run[rr] - m_new);
             m_run[rr] = m_new;
+            m_sub[rr] = P_BIAS_LOG2 - m_new;            // probabilities come out times 64
         }
+        if (__any_sync(0xffffffffu, alpha[0] != 1.0f || alpha[1] != 1.0f)) {
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-            o[i][0] *= alpha[0];
-            o[i][1] *= alpha[0];
-            o[i][2] *= alpha[1];
-            o[i][3] *= alpha[1];
+            for (int i = 0; i < D / 8; ++i) {
+                o[i][0] *= alpha[0];
+                o[i][1] *= alpha[0];
+                o[i][2] *= alpha[1];
+                o[i][3] *= alpha[1];
+            }
         }
         // ---- O += P V, sixteen tokens at a time.  P enters the tensor core as fp16 hi + lo halves (two
         // products), which keeps ~22 bits of it: a single fp16 rounding of P alone would cost ~1e-3 of
@@ -276,12 +410,10 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int rr = e >> 1;
-                    pv[e] = s[n][e] > 0.5f * NEG_BIG ? exp2f(s[n][e] - m_run[rr]) : 0.f;
+                    pv[e] = s[n][e] > NEG_LIVE ? ex2(fmaf(s[n][e], P.scale_log2, m_sub[rr])) : 0.f;
                 }
                 ls[0] += pv[0] + pv[1];
                 ls[1] += pv[2] + pv[3];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) pv[e] *= P_BIAS;
                 const uint32_t h01 = pack_h2(pv[0], pv[1]), h23 = pack_h2(pv[2], pv[3]);
                 const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&h01));
                 const float2 f23 = __half22float2(*reinterpret_cast<const __half2*>(&h23));
@@ -295,8 +427,8 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
                 uint32_t bv[4];
                 ldsm_x4_t(v_addr + (k2 * 16 * PITCH) * 2 + n2 * 32, bv);
                 mma16816(o[2 * n2], ph, bv[0], bv[1]);
-                mma16816(o[2 * n2], pl, bv[0], bv[1]);
                 mma16816(o[2 * n2 + 1], ph, bv[2], bv[3]);
+                mma16816(o[2 * n2], pl, bv[0], bv[1]);
                 mma16816(o[2 * n2 + 1], pl, bv[2], bv[3]);
             }
         }
@@ -306,27 +438,73 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
             ls[rr] += __shfl_xor_sync(0xffffffffu, ls[rr], 2);
             l_run[rr] = l_run[rr] * alpha[rr] + ls[rr];
         }
+        __syncthreads();                                // the tile has been read: its buffer may be refilled
     }
 
-    // ---- normalise and store: out (B, S, H, D)
+    if (P.splits == 1) {
+        // ---- normalise and store: out (B, S, H, D)
+#pragma unroll
+        for (int rr = 0; rr < 2; ++rr) {
+            if (!row_live[rr]) continue;
+            const int r = warp * 16 + g + 8 * rr;
+            const int tl = r >> gp_shift, hg = r & (P.Gp - 1);
+            const float inv = l_run[rr] > 0.f ? 1.0f / l_run[rr] : 0.f;
+            const int64_t base = ((static_cast<int64_t>(b) * P.S + tok0 + tl) * P.H + kvh * P.G + hgrp * 8 + hg) * D;
+#pragma unroll
+            for (int i = 0; i < D / 8; ++i)
+                store_out(P.out, P.q_dtype, base + 8 * i + 2 * t, o[i][2 * rr] * inv, o[i][2 * rr + 1] * inv);
+        }
+        return;
+    }
+    // ---- merge the cluster's partial results: every CTA leaves its own in its shared memory and finishes ROWS / splits rows
+    float* Os = reinterpret_cast<float*>(tiles);        // [row][D]
 #pragma unroll
     for (int rr = 0; rr < 2; ++rr) {
-        if (!row_live[rr]) continue;
         const int r = warp * 16 + g + 8 * rr;
-        const int tl = r >> gp_shift, hg = r & (P.Gp - 1);
-        const float inv = l_run[rr] > 0.f ? 1.0f / (P_BIAS * l_run[rr]) : 0.f;
-        const int64_t base = ((static_cast<int64_t>(b) * P.S + tok0 + tl) * P.H + kvh * P.G + hgrp * 8 + hg) * D;
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i)
-            store_out(P.out, P.q_dtype, base + 8 * i + 2 * t, o[i][2 * rr] * inv, o[i][2 * rr + 1] * inv);
+        for (int i = 0; i < D / 8; ++i) *reinterpret_cast<float2*>(Os + r * D + 8 * i + 2 * t) = make_float2(o[i][2 * rr], o[i][2 * rr + 1]);
+        if (t == 0) {
+            Ms[r] = m_run[rr];
+            Ls[r] = l_run[rr];
+        }
     }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int rows_here = ROWS / P.splits, r0 = split * rows_here;
+    for (int i = threadIdx.x; i < rows_here * (D / 4); i += WARPS * 32) {
+        const int r = r0 + i / (D / 4), c = (i % (D / 4)) * 4;
+        const int tl = r >> gp_shift, hg = r & (P.Gp - 1);
+        if (tok0 + tl >= P.S || hg >= heads_here) continue;
+        float top = NEG_BIG;
+        for (int k = 0; k < P.splits; ++k) top = fmaxf(top, peer_f32(Ms + r, k));
+        float l = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < P.splits; ++k) {
+            const float w = ex2(peer_f32(Ms + r, k) - top);
+            const float4 v = peer_f32x4(Os + r * D + c, k);
+            l = fmaf(w, peer_f32(Ls + r, k), l);
+            acc.x = fmaf(w, v.x, acc.x);
+            acc.y = fmaf(w, v.y, acc.y);
+            acc.z = fmaf(w, v.z, acc.z);
+            acc.w = fmaf(w, v.w, acc.w);
+        }
+        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        const int64_t base = ((static_cast<int64_t>(b) * P.S + tok0 + tl) * P.H + kvh * P.G + hgrp * 8 + hg) * D + c;
+        store_out(P.out, P.q_dtype, base, acc.x * inv, acc.y * inv);
+        store_out(P.out, P.q_dtype, base + 2, acc.z * inv, acc.w * inv);
+    }
+    // nobody's shared memory goes away while a peer still reads it
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// CTAs below which the key range is split over a cluster: two per SM are resident, and a short chunk's few CTAs each walk
+// the whole history (77 tokens behind 1500, 32/8 heads: 40 CTAs of 25 tiles, 162 us of which one CTA's chain was all).
+constexpr int MIN_CTAS = 2 * 148;
+
 template <int LAYOUT, int D>
-static int launch_one(const Params& P, cudaStream_t st) {
+static int launch_one(Params& P, cudaStream_t st) {
     static bool configured[64] = {};
     auto kern = attn_chunk_kernel<LAYOUT, D>;
-    constexpr int SMEM = 3 * ROWS * (D + 8) * 2;
+    constexpr int SMEM = Smem<LAYOUT, D>::BYTES;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!configured[dev]) {
@@ -335,14 +513,31 @@ static int launch_one(const Params& P, cudaStream_t st) {
         configured[dev] = true;
     }
     const int TQ = ROWS / P.Gp;
-    const dim3 grid((P.S + TQ - 1) / TQ, P.KV_H * P.HG, P.B);
-    const cudaError_t e = launch_pdl(kern, grid, dim3(WARPS * 32), SMEM, st, P);
+    const int64_t ctas = static_cast<int64_t>((P.S + TQ - 1) / TQ) * P.KV_H * P.HG * P.B;
+    // the history's length is known on the device only; the cache's bounds it (four tiles per CTA at least)
+    P.splits = 1;
+    while (P.splits < 8 && ctas * P.splits < MIN_CTAS && P.kv.S_max >= 2 * P.splits * 4 * KT) P.splits *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((P.S + TQ - 1) / TQ * P.splits, P.KV_H * P.HG, P.B);
+    cfg.blockDim = dim3(WARPS * 32);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = P.splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = P.splits > 1 ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P);
     if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
     return check_launch();
 }
 
 template <int LAYOUT>
-static int launch_d(const Params& P, int D, cudaStream_t st) {
+static int launch_d(Params& P, int D, cudaStream_t st) {
     switch (D) {
         case 64: return launch_one<LAYOUT, 64>(P, st);
         case 128: return launch_one<LAYOUT, 128>(P, st);
@@ -421,6 +616,7 @@ extern "C" int alloyb_attn_chunk(int layout, const void* q, int64_t q_batch_stri
     const float sc = scale > 0.f ? scale : 1.0f / sqrtf(static_cast<float>(D));
     P.scale_log2 = sc * 1.4426950408889634f;
     P.status = reinterpret_cast<int*>(status);
+    P.pool_aligned = reinterpret_cast<uintptr_t>(k0) % 16 == 0;
     cudaStream_t st = as_stream(stream);
     switch (layout) {
         case ALLOYB_KV_F16: return ac::launch_d<ALLOYB_KV_F16>(P, D, st);

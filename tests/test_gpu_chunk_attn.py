@@ -182,3 +182,50 @@ def test_chunk_attention_errors():
     torch.ops.alloy.attention_cache(q, nk, nk, torch.tensor([31], device=DEV), cache, cache, 0.125)
     assert ops.attn_status(ops.attn_workspace(torch.device(DEV, 0), 1, 4, d)) & 1
     ops._workspaces.clear()
+
+
+@pytest.mark.parametrize("layout,b,kv_h,group,d,start,chunk", [
+    ("f16", 1, 2, 4, 128, 1900, 3), ("f16", 1, 1, 1, 64, 0, 2), ("q8", 2, 1, 7, 128, 700, 40), ("q8", 1, 3, 4, 64, 1000, 18),
+    ("paged", 1, 2, 4, 128, 1999, 17), ("paged", 1, 1, 8, 256, 515, 2)])
+def test_chunk_over_a_split_history(layout, b, kv_h, group, d, start, chunk):
+    """Few rows: the key range is split over a cluster whose CTAs merge through distributed shared memory; some CTAs get
+    no tile, or none that a row may see."""
+    rng = np.random.default_rng([b, d, start, chunk])
+    h, n, s_max = kv_h * group, start + chunk, 2048
+    k, v = synth.kv_rows(rng, (b, kv_h, n, d)), synth.kv_rows(rng, (b, kv_h, n, d))
+    q = synth.activations(rng, b * h * chunk, d).reshape(b, h, chunk, d)
+    nk, nv = _dev(k[:, :, start:]), _dev(v[:, :, start:])
+    if layout == "f16":
+        caches = [torch.zeros((b, kv_h, s_max, d), dtype=torch.float16, device=DEV) for _ in range(2)]
+        for c, rows in zip(caches, (k, v)):
+            c[:, :, :start] = _dev(rows[:, :, :start])
+        out = torch.ops.alloy.attention_cache(_dev(q), nk, nv, torch.tensor([start], device=DEV), *caches, -1.0)
+        kr, vr = k.astype(np.float32), v.astype(np.float32)
+    else:
+        (kc, ks), (vc, vs) = O.kv_quantize_q8_0(k), O.kv_quantize_q8_0(v)
+        kr, vr = _deq16(kc, ks), _deq16(vc, vs)
+        if layout == "q8":
+            caches = kv.alloc_quantized_kv(b, kv_h, s_max, d, DEV)
+            for c, rows in zip(caches, (kc, ks, vc, vs)):
+                c[:, :, :start] = _dev(rows[:, :, :start])
+            out = torch.ops.alloy.attention_cache_q8(_dev(q), nk, nv, torch.tensor([start], device=DEV), *caches)
+        else:
+            outs = []
+            for shift in (0, 2):         # a pool that starts off a 16-byte boundary gives the same bytes
+                store = kv.PagedKVPool(s_max // 16, kv_h, d, b, s_max // 16, DEV, free_order=rng.permutation(s_max // 16).tolist())
+                if shift:
+                    raw = torch.zeros(store.pool.numel() + 16, dtype=torch.uint8, device=DEV)
+                    store.pool = raw[shift:shift + store.pool.numel()].view(store.pool.shape)
+                store.reserve(0, s_max)
+                pages = torch.zeros((s_max // 16, 2, kv_h, 16, d // 32 * 34), dtype=torch.uint8)
+                for j, (codes, scales) in enumerate(((kc, ks), (vc, vs))):
+                    rows = np.zeros((kv_h, s_max, d // 32 * 34), np.uint8)
+                    rows[:, :start] = O.kv_pack_blocks(codes, scales)[0, :, :start]
+                    pages[:, j] = torch.from_numpy(rows).view(kv_h, -1, 16, d // 32 * 34).transpose(0, 1)
+                store.pool[torch.tensor(store.pages_of(0), device=DEV)] = pages.to(DEV)
+                outs.append(torch.ops.alloy.attention_cache_q8_paged(_dev(q), nk, nv, torch.tensor([start], dtype=torch.int32, device=DEV),
+                                                                     store.page_table, store.pool))
+            assert torch.equal(*outs)
+            out = outs[0]
+    ref = np.stack([O.attention_chunk_ref(kr[i], vr[i], q[i].astype(np.float64), start) for i in range(b)])
+    assert_close(to_np(out), ref, torch.float16, f"split history {layout}")
