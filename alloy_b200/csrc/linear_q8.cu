@@ -1,4 +1,5 @@
-// Q8_0 dequant-GEMV for 1..4 tokens per pass (more tokens: more passes), plain and gate/up fused.
+// Q8_0 dequant-GEMV for 1..4 tokens per pass (more tokens: more passes), plain and gate/up fused.  (One token and K from
+// 4096 to 16384: q8_gemv_one_kernel, further down.)
 //
 // Weights arrive in the reference's normalised pair (server/gguf/quant.py:497-521): int8 codes
 // (N, K) and fp16 scales (N, K/32), w = scale * code; 1.0625 bytes per weight, so the kernel is a
@@ -159,6 +160,196 @@ __global__ void __launch_bounds__(WARPS * 32, MTOK == 1 ? 2 : 1) q8_gemv_kernel(
         }
 }
 
+// ---- one token, K up to 16384: the token stays in registers.
+//
+// The kernel above spends its time on instructions (4.4 per code: activations converted again for every four rows) and on
+// its waves (14336 gate/up rows: 896 CTAs, 3.03 waves of 296).  Here the eight warps of a CTA split K -- a lane keeps its 16
+// activations of up to NS 512-wide slices as fp32 pairs for the whole launch -- and walk the CTA's share of the rows
+// together, RB rows (or gate and up rows) at a time with the next step's loads in flight.  Codes become fp32 pairs by two
+// byte permutes and the two-wide add, products run on the two-wide FMA: 9 instructions per four codes.  The lanes' sums of
+// RB rows are folded together (9 shuffles for 8 rows); the warps' sums meet in shared memory once, at the end.
+__device__ __forceinline__ uint64_t pair(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+constexpr int SLICE = 512;           // 32 lanes x 16 codes
+constexpr int MAX_SLICES = 4;        // per warp
+
+template <typename XT, bool GATED, int NS, int RB>
+__global__ void __launch_bounds__(WARPS * 32, 2) q8_gemv_one_kernel(const Params P) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float part[];                 // [row of the CTA][matrix][warp]
+    constexpr int NM = GATED ? 2 : 1, R = RB / NM;                // rows of each matrix per step
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int K = P.K, nblk = K / Q8_BLOCK, slices = K / SLICE;
+    const int units = (P.N + R - 1) / R;
+    const int u0 = static_cast<int>(static_cast<int64_t>(units) * blockIdx.x / gridDim.x);
+    const int u1 = static_cast<int>(static_cast<int64_t>(units) * (blockIdx.x + 1) / gridDim.x);
+    const int mine = (slices - warp + WARPS - 1) / WARPS;         // this warp's slices: warp, warp + 8, ...
+
+    struct Step {
+        uint4 c[RB];
+        __half s[RB];
+    };
+    // step i: rows u0 * R + (i / NS) * R .., slice i % NS (of `mine`; the others are skipped)
+    auto load = [&](int unit, int sl, Step& o) {
+        const int k = (warp + sl * WARPS) * SLICE + lane * 16;
+#pragma unroll
+        for (int a = 0; a < NM; ++a)
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int64_t row = min(unit * R + r, P.N - 1);   // tail rows re-read the last row
+                o.c[a * R + r] = __ldg(reinterpret_cast<const uint4*>(P.w[a] + row * K + k));
+                o.s[a * R + r] = __ldg(P.s[a] + row * nblk + k / Q8_BLOCK);
+            }
+    };
+    // weights do not depend on the previous kernel
+    Step even, odd;
+    if (u0 < u1 && mine > 0) load(u0, 0, even);
+    pdl_wait();
+    uint64_t x[NS][8];
+#pragma unroll
+    for (int sl = 0; sl < NS; ++sl) {
+        const XT* xp = static_cast<const XT*>(P.x) + (warp + (sl < mine ? sl : 0) * WARPS) * SLICE + lane * 16;
+        XT v[16];
+#pragma unroll
+        for (int q = 0; q < 16 * static_cast<int>(sizeof(XT)) / 16; ++q)
+            reinterpret_cast<uint4*>(v)[q] = mine > 0 ? __ldg(reinterpret_cast<const uint4*>(xp) + q) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[sl][e] = pair(to_f32<XT>(v[2 * e]), to_f32<XT>(v[2 * e + 1]));
+    }
+    const uint64_t unbias = pair(-8388736.0f, -8388736.0f);      // -(2^23 + 128)
+    float acc[RB];
+    auto compute = [&](const Step& o, const uint64_t (&xs)[8], bool first) {
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+            const uint32_t wv[4] = {o.c[j].x, o.c[j].y, o.c[j].z, o.c[j].w};
+            uint64_t sum = pair(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t u = wv[q] ^ 0x80808080u;
+                constexpr uint32_t MAGIC = 0x4B000000u;
+                sum = fma2(add2(pair(__uint_as_float(prmt(u, MAGIC, 0x7650u)), __uint_as_float(prmt(u, MAGIC, 0x7651u))), unbias), xs[2 * q], sum);
+                sum = fma2(add2(pair(__uint_as_float(prmt(u, MAGIC, 0x7652u)), __uint_as_float(prmt(u, MAGIC, 0x7653u))), unbias), xs[2 * q + 1], sum);
+            }
+            float a, b;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(sum));
+            acc[j] = fmaf(__half2float(o.s[j]), a + b, first ? 0.f : acc[j]);
+        }
+    };
+    auto finish = [&](int unit) {
+        // fold: after the steps with lane distance 16, 8, (4) a lane holds one row's sum over its lane group
+        float v[RB];
+#pragma unroll
+        for (int j = 0; j < RB; ++j) v[j] = acc[j];
+        int idx = 0;
+#pragma unroll
+        for (int h = RB / 2, d = 16; h >= 1; h /= 2, d /= 2) {
+            const bool up = (lane & d) != 0;
+            idx = idx * 2 + (up ? 1 : 0);
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const float give = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+                v[j] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+            }
+        }
+        constexpr int LEFT = 32 / RB;                             // lanes that share a row
+#pragma unroll
+        for (int d = LEFT / 2; d >= 1; d /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], d);
+        if ((lane & (LEFT - 1)) == 0) part[((unit - u0) * RB + idx) * WARPS + warp] = v[0];
+    };
+    // (every warp has work: slices >= WARPS, see the caller)
+    const int steps = (u1 - u0) * mine;
+    int unit = u0, sl = 0, l_unit = u0, l_sl = 0;
+    auto advance = [&](int& un, int& s) {
+        if (++s == mine) {
+            s = 0;
+            ++un;
+        }
+    };
+    auto run = [&](Step& cur, Step& next, bool more) {
+        advance(l_unit, l_sl);
+        if (more) load(l_unit, l_sl, next);                       // in flight while this step is computed
+        if (NS == 1) {
+            compute(cur, x[0], true);
+        } else {
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                if (s == sl) compute(cur, x[s], s == 0);
+        }
+        if (sl == mine - 1) finish(unit);
+        advance(unit, sl);
+    };
+    for (int i = 0; i < steps; i += 2) {
+        run(even, odd, i + 1 < steps);
+        if (i + 1 < steps) run(odd, even, i + 2 < steps);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < (u1 - u0) * R; i += WARPS * 32) {
+        const int un = i / R, r = i - un * R, row = (u0 + un) * R + r;
+        if (row >= P.N) continue;
+        float v = 0.f, u = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            v += part[(un * RB + r) * WARPS + w];
+            if (GATED) u += part[(un * RB + R + r) * WARPS + w];
+        }
+        XT* y = static_cast<XT*>(P.y);
+        if (GATED) {
+            const float a = (P.act == ALLOYB_ACT_SILU) ? act_silu(v) : act_gelu_tanh(v);
+            y[row] = from_f32<XT>(a * u);
+        } else {
+            XT out = from_f32<XT>(v);
+            if (P.residual) out = from_f32<XT>(to_f32<XT>(static_cast<const XT*>(P.residual)[row]) + to_f32<XT>(out));
+            y[row] = out;
+        }
+    }
+}
+
+template <typename XT, bool GATED, int NS, int RB>
+static int launch_one_ns(const Params& P, cudaStream_t st) {
+    static bool configured[64] = {};
+    static int sm_count[64] = {};
+    auto kern = q8_gemv_one_kernel<XT, GATED, NS, RB>;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (!configured[dev]) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
+        configured[dev] = true;
+    }
+    const int units = (P.N + RB / (GATED ? 2 : 1) - 1) / (RB / (GATED ? 2 : 1));
+    const int grid = units < 2 * sm_count[dev] ? units : 2 * sm_count[dev];
+    const size_t smem = static_cast<size_t>((units + grid - 1) / grid) * RB * WARPS * 4;
+    if (smem > 100 * 1024) return ALLOYB_NOT_TAKEN;
+    const cudaError_t e = launch_pdl(kern, dim3(grid), dim3(WARPS * 32), smem, st, P);
+    if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
+    return check_launch();
+}
+// Every warp has at least one slice from K = 4096 on; one slice each leaves the registers for eight rows at a time.
+template <typename XT, bool GATED>
+static int launch_one(const Params& P, cudaStream_t st) {
+    const int slices = P.K / SLICE, ns = (slices + WARPS - 1) / WARPS;
+    if (slices < WARPS || ns > MAX_SLICES) return ALLOYB_NOT_TAKEN;
+    switch (ns) {
+        case 1: return launch_one_ns<XT, GATED, 1, 8>(P, st);
+        case 2: return launch_one_ns<XT, GATED, 2, 4>(P, st);
+        default: return launch_one_ns<XT, GATED, 4, 4>(P, st);
+    }
+}
+
 template <typename XT, bool GATED, int MTOK>
 static int launch_m(const Params& P, cudaStream_t st) {
     static bool configured[64] = {};
@@ -180,7 +371,11 @@ static int launch_m(const Params& P, cudaStream_t st) {
 
 template <typename XT, bool GATED>
 static int launch(const Params& P, cudaStream_t st) {
-    return P.M == 1 ? launch_m<XT, GATED, 1>(P, st) : launch_m<XT, GATED, MT>(P, st);
+    if (P.M == 1) {
+        const int rc = launch_one<XT, GATED>(P, st);
+        return rc == ALLOYB_NOT_TAKEN ? launch_m<XT, GATED, 1>(P, st) : rc;
+    }
+    return launch_m<XT, GATED, MT>(P, st);
 }
 
 }  // namespace q8

@@ -395,3 +395,23 @@ def test_no_device_error_recorded():
     """No kernel of this module ran out a bounded wait."""
     from alloy_b200 import _lib
     assert _lib.load().alloyb_device_error(0) == 0
+
+
+@pytest.mark.parametrize("n,k", [(1, 4096), (37, 4608), (1203, 4096), (130, 8192), (64, 16384), (50, 16896)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+def test_q8_0_one_token(n, k, dt):
+    """One token against Q8_0 rows of 4096 weights and more: the token in registers, K split over the warps (16896: too
+    long for that, the general kernel)."""
+    rng = np.random.default_rng([n, k])
+    (gc, gs), (uc, us) = (O.split_q8_0(synth.q8_0_wire(rng, n, k)) for _ in range(2))
+    x = torch.from_numpy(synth.activations(rng, 1, k, np.float32)).to(dt)
+    g = x.double().numpy() @ O.dequant_q8_0(gc, gs).astype(np.float64).T
+    u = x.double().numpy() @ O.dequant_q8_0(uc, us).astype(np.float64).T
+    xd, w = x.to(DEV), [_dev(a) for a in (gc, gs, uc, us)]
+    assert_close(to_np(torch.ops.alloy.gguf_q8_0_mm(xd, *w[:2])), g, dt, f"q8_0 {n}x{k}")
+    assert_close(to_np(torch.ops.alloy.gguf_q8_0_silu(xd, *w)), O.silu(g) * u, dt, f"q8_0 gated {n}x{k}")
+    if n > 1:
+        res = torch.from_numpy(synth.activations(rng, 1, n, np.float32)).to(dt).to(DEV)
+        y = torch.ops.alloy.linear_residual(xd, w[0], w[1], res, "q8_0")
+        plain = torch.ops.alloy.gguf_q8_0_mm(xd, *w[:2])
+        assert torch.equal(y, (res.float() + plain.float()).to(dt))
