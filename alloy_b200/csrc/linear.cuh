@@ -34,6 +34,15 @@ int try_gemv_stream(const void* x, int M, int K, int dtype, const WeightSeg* seg
 int try_gemv_stream_mixed(const void* x, int M, int K, int dtype, const WeightSeg* seg, int n_seg, const void* residual,
                           const void* norm_w, float eps, cudaStream_t stream);
 int gemv_stream_device_error(int clear);
+// A few fp16 tokens (2..SKINNY_MAX_M) against Q4_K / Q6_K matrices (linear_skinny.cu).  Up to 16 tokens it takes Q4_K only,
+// K = 2048 / 4096 / 8192 (the tokens' fragments then live in registers) and more than two tiles per SM: at 16 tokens gate/up
+// 14336 x 4096 takes 29.8 us against 45.5 with the tokens-as-columns kernel, 4096 x 4096 9.9 against 8.5.  From 17 tokens on
+// it takes every shape: 24 tokens 46 against 87 us, 10.8 against 13.0, Q6_K 4096 x 14336 35.5 against 41.6.  From 28 on the
+// tcgen05 GEMM's definition (weights rounded to the activation type) holds.
+constexpr int SKINNY_MAX_M = 27;
+int try_linear_skinny(const void* x, int M, int K, int dtype, const WeightSeg* seg, int n_seg, bool gated, int act,
+                      const void* residual, cudaStream_t st);
+int linear_skinny_device_error(int clear);
 int decode_layer_device_error(int clear);
 
 // Q8_0 streaming GEMV (1..63 tokens, four per pass), plain (w1 == nullptr) or gate/up fused.
