@@ -15,6 +15,8 @@
 // mma.sync.m16n8k16 (fp16 operands, fp32 accumulation) with ldmatrix fragment loads; the softmax
 // is the usual online one in the exp2 frame; P enters the second product as fp16 hi + lo halves.
 //
+// (fp16 queries over an fp16 cache at head_dim 128 with many rows: attn_prefill.cu.)
+//
 // What bounds it: a long prompt, the mma.sync pipe (three products of 64 x 64 x D per tile); a short chunk behind a long
 // history, the length of the chain of tiles.  So the next tile's K and V are copied (cp.async) while this one is computed
 // -- q8_0 caches: their raw bytes, which are expanded to the fp16 tile from shared memory --, and when the rows alone
@@ -548,6 +550,10 @@ static int launch_d(Params& P, int D, cudaStream_t st) {
 
 }  // namespace ac
 
+// defined in attn_prefill.cu
+int try_attn_prefill(const void* q, int64_t q_bs, int64_t q_hs, int64_t q_ts, int q_dtype, const KVPtrs& kv, const int32_t* start,
+                     int start_count, void* out, int B, int H, int KV_H, int dim, int n_tokens, float scale_log2, int* status, cudaStream_t st);
+
 // defined in kv.cu (shares the block quantiser with the one-token append)
 int launch_kv_write_range(int layout, const void* new_k, const void* new_v, int64_t sb, int64_t sh, int64_t stok,
                           const KVPtrs& kv, const int32_t* start, int start_count, int B, int KV_H, int D,
@@ -618,6 +624,11 @@ extern "C" int alloyb_attn_chunk(int layout, const void* q, int64_t q_batch_stri
     P.status = reinterpret_cast<int*>(status);
     P.pool_aligned = reinterpret_cast<uintptr_t>(k0) % 16 == 0;
     cudaStream_t st = as_stream(stream);
+    if (layout == ALLOYB_KV_F16) {
+        const int taken = try_attn_prefill(q, q_batch_stride, q_head_stride, q_tok_stride, q_dtype, P.kv, start, start_count, out, B, H, KV_H,
+                                           D, n_tokens, P.scale_log2, P.status, st);
+        if (taken != ALLOYB_NOT_TAKEN) return taken;
+    }
     switch (layout) {
         case ALLOYB_KV_F16: return ac::launch_d<ALLOYB_KV_F16>(P, D, st);
         case ALLOYB_KV_Q8_SPLIT: return ac::launch_d<ALLOYB_KV_Q8_SPLIT>(P, D, st);

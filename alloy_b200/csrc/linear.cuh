@@ -44,6 +44,7 @@ int try_linear_skinny(const void* x, int M, int K, int dtype, const WeightSeg* s
                       const void* residual, cudaStream_t st);
 int linear_skinny_device_error(int clear);
 int decode_layer_device_error(int clear);
+int attn_prefill_device_error(int clear);
 
 // Q8_0 streaming GEMV (1..63 tokens, four per pass), plain (w1 == nullptr) or gate/up fused.
 int try_q8_gemv(const void* x, int M, int K, int dtype, const void* w0, const void* s0, const void* w1, const void* s1,

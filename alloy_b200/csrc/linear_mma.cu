@@ -828,7 +828,7 @@ extern "C" int alloyb_device_error(int clear) {
     if (e != cudaSuccess) { alloyb::set_cuda_error(e); return ALLOYB_E_CUDA; }
     const int v_tc = alloyb::gemm_tc_device_error(clear) | alloyb::attn_mma_device_error(clear) |
                      alloyb::gemv_stream_device_error(clear) | alloyb::linear_skinny_device_error(clear) |
-                     alloyb::decode_layer_device_error(clear);
+                     alloyb::attn_prefill_device_error(clear) | alloyb::decode_layer_device_error(clear);
     if (clear && v) {
         const int z = 0;
         e = cudaMemcpyToSymbol(alloyb::g_device_error, &z, sizeof(int));

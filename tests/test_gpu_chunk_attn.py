@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from alloy_b200 import kv, ops, synth
+from alloy_b200 import _lib, kv, ops, synth
 from oracle import blocks as O
 from tests._util import assert_close, to_np
 
@@ -229,3 +229,25 @@ def test_chunk_over_a_split_history(layout, b, kv_h, group, d, start, chunk):
             out = outs[0]
     ref = np.stack([O.attention_chunk_ref(kr[i], vr[i], q[i].astype(np.float64), start) for i in range(b)])
     assert_close(to_np(out), ref, torch.float16, f"split history {layout}")
+
+
+@pytest.mark.parametrize("b,kv_h,group,start,chunk", [(1, 8, 4, 0, 800), (2, 8, 7, 130, 321), (1, 32, 1, 1, 700), (3, 4, 16, 300, 133),
+                                                      (1, 96, 2, 127, 129), (1, 96, 1, 2000, 2)])
+def test_long_chunk_on_the_tensor_cores(b, kv_h, group, start, chunk):
+    """Enough rows for the tcgen05 kernel: tiles of 256 rows and 128 keys with ragged ends, padded head groups, scores that
+    make the maximum climb, and a cache whose unused rows hold NaN."""
+    gen = torch.Generator(device=DEV).manual_seed(b * 1000 + chunk)
+    h, d, n, s_max = kv_h * group, 128, start + chunk, start + chunk + 150
+    rows = [torch.randn((b, kv_h, n, d), device=DEV, generator=gen).half() for _ in range(2)]
+    rows[0] *= torch.linspace(0.2, 6.0, n, device=DEV).half().view(n, 1)         # later keys score higher
+    q = torch.randn((b, h, chunk, d), device=DEV, generator=gen).half()
+    caches = [torch.full((b, kv_h, s_max, d), float("nan"), dtype=torch.float16, device=DEV) for _ in range(2)]
+    for c, r in zip(caches, rows):
+        c[:, :, :start] = r[:, :, :start]
+    new = [r[:, :, start:].transpose(1, 2).contiguous().transpose(1, 2) for r in rows]
+    out = torch.ops.alloy.attention_cache(q, *new, torch.tensor([start], device=DEV), *caches, -1.0)
+    s = q.double().unflatten(1, (kv_h, group)) @ rows[0].double().unsqueeze(2).transpose(-1, -2) / np.sqrt(d)
+    seen = torch.arange(n, device=DEV) <= start + torch.arange(chunk, device=DEV).unsqueeze(1)
+    ref = (s.masked_fill(~seen, -np.inf).softmax(-1) @ rows[1].double().unsqueeze(2)).flatten(1, 2)
+    assert_close(to_np(out), ref.cpu().numpy(), torch.float16, "long chunk")
+    assert _lib.load().alloyb_device_error(1) == 0
