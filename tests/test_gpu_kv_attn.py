@@ -425,3 +425,20 @@ def test_rope_attention_decode_positions_and_fallback(pos0):
         got = ops.rope_attention_decode(q, nk, nv, pos, inv, k_cache=c2[0], v_cache=c2[1])
         assert torch.equal(c1[0], c2[0]) and torch.equal(c1[1], c2[1])
         assert torch.equal(want, got)
+
+
+@pytest.mark.parametrize("b,kv_h,group,pos", [(1, 2, 4, 15), (3, 1, 8, 16), (2, 8, 4, 63), (2, 2, 1, 200), (20, 8, 4, 130), (1, 1, 7, 5000)])
+def test_attention_f16_tiles_through_the_ring(b, kv_h, group, pos):
+    """The fp16 cache's tiles pass through a ring of two per warp: lengths around a tile, around the four warps' tiles and
+    around a CTA's share, with NaN in the rows past the last one."""
+    gen = torch.Generator(device=DEV).manual_seed(pos)
+    h, d, s_max = kv_h * group, 128, pos + 40
+    k, v = (torch.randn((b, kv_h, pos + 1, d), device=DEV, generator=gen).half() for _ in range(2))
+    q = torch.randn((b, h, 1, d), device=DEV, generator=gen).half()
+    caches = [torch.full((b, kv_h, s_max, d), float("nan"), dtype=torch.float16, device=DEV) for _ in range(2)]
+    for c, r in zip(caches, (k, v)):
+        c[:, :, :pos] = r[:, :, :pos]
+    out = torch.ops.alloy.attention_cache(q, k[:, :, pos:], v[:, :, pos:], torch.tensor([pos], device=DEV), *caches, -1.0)
+    s = q.double().unflatten(1, (kv_h, group)) @ k.double().unsqueeze(2).transpose(-1, -2) / np.sqrt(d)
+    ref = (s.softmax(-1) @ v.double().unsqueeze(2)).flatten(1, 2)
+    assert_close(to_np(out), ref.cpu().numpy(), torch.float16, f"f16 ring {b} {pos}")
