@@ -87,6 +87,9 @@ int alloyb_dequant_q5_0(const void* qweight, const void* qhigh, const void* scal
  * reference's batched ops do by concatenating rows
  * (torch/ops/linalg.py:555-669, torch/custom_ops.py:50-52, :100-102, :106-108).
  *
+ * Packed weights and their scales count as constants: the kernels request them while the kernel before them in
+ * the stream is still draining (programmatic dependent launch); activations, residuals and outputs wait for it.
+ *
  * M routing inside the library replaces torch/ops/linalg.py:462-497 (Q4_K),
  * :726-739 (Q6_K), :346-401 (Q8_0): small M runs the bandwidth-bound
  * dequant-GEMV family (metal/std/quant.py:1356-1453 dot_q4_k_v2, :2201-2277
