@@ -1,5 +1,6 @@
-// Dequant-GEMV / skinny GEMM for 2..128 tokens (32 per pass) and for the one-token shapes the
-// persistent streaming kernel (linear_stream.cu) does not take (bf16, K not a multiple of 1024).
+// Dequant-GEMV / skinny GEMM for a few tokens: fp16 up to 16 (what linear_skinny.cu leaves: Q6_K, matrices of at most two
+// tiles per SM, other K), bf16 up to 27, and the one-token shapes the persistent streaming kernel (linear_stream.cu) does
+// not take (bf16, K not a multiple of 1024).
 //
 // Why tensor cores on a memory-bound op: at HBM speed a B200 streams ~11.5e12
 // Q4_K weights per second but issues only ~1.1e12 warp instructions per second,
@@ -711,7 +712,10 @@ static int launch_mma_nt(MmaParams& P, int grid, int stage_rows_bytes, cudaStrea
     switch (NTt) {
         case 1: return launch_mma<XT, RT, 1>(P, grid, smem, st);
         case 2: return launch_mma<XT, RT, 2>(P, grid, smem, st);
-        default: return launch_mma<XT, RT, 4>(P, grid, smem, st);
+        default:
+            // fp16 calls of 17 tokens and more went to linear_skinny.cu (same alignment rules) or the GEMM
+            if constexpr (std::is_same<XT, __half>::value) return ALLOYB_NOT_TAKEN;
+            else return launch_mma<XT, RT, 4>(P, grid, smem, st);
     }
 }
 
