@@ -95,8 +95,10 @@ _BLOCK_BYTES = {_lib.Q4_K: 144, _lib.Q6_K: 210}
 
 
 _launches = 0
-# The current stream of the current device, without building a Stream object for every call.
-_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch.cuda.current_device
+# The current stream of a device, without building a Stream object for every call where torch offers that (a build without
+# CUDA does not).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+_current_device = torch.cuda.current_device
 
 
 def launch_count() -> int:

@@ -5,6 +5,7 @@ validation behaves like the reference's."""
 import os
 import pathlib
 import re
+import subprocess
 import sys
 
 import numpy as np
@@ -202,3 +203,15 @@ def test_kv_format_and_page_pool_host_logic():
     small = kv.PagedKVPool(2, 2, 128, 1, 3, "cpu")
     with pytest.raises(MemoryError):
         small.reserve(0, 48)
+
+
+def test_ops_import_without_a_cuda_build_of_torch():
+    """A torch build without CUDA has no raw-stream query: the module still imports there and its Meta kernels work."""
+    code = ("import torch\n"
+            "del torch._C._cuda_getCurrentRawStream\n"
+            "import alloy_b200\n"
+            "y = torch.ops.alloy.gguf_q4_k_mm(torch.empty(3, 512, device='meta', dtype=torch.float16),\n"
+            "                                 torch.empty(40, 288, device='meta', dtype=torch.uint8))\n"
+            "assert y.shape == (3, 40)\n")
+    run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr
