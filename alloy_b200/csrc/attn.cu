@@ -378,7 +378,11 @@ static int attn_decode_validate(int layout, const void* q, int q_dtype, const vo
         return ALLOYB_E_SHAPE;
     if (pos_count != 1 && pos_count != B) return ALLOYB_E_SHAPE;
     if (q_dtype != ALLOYB_F16 && q_dtype != ALLOYB_BF16 && q_dtype != ALLOYB_F32) return ALLOYB_E_DTYPE;
-    if (layout == ALLOYB_KV_F16) { if (!v0) return ALLOYB_E_NULL; }
+    if (layout == ALLOYB_KV_F16) {
+        if (!v0) return ALLOYB_E_NULL;
+        // K rows are read 16 bytes at a time; V rows at least 8 (head_dim 128) or element by element
+        if (reinterpret_cast<uintptr_t>(k0) % 16 || reinterpret_cast<uintptr_t>(v0) % (D == 128 ? 8 : 2)) return ALLOYB_E_ALIGN;
+    }
     else if (layout == ALLOYB_KV_Q8_SPLIT) { if (!k1 || !v0 || !v1) return ALLOYB_E_NULL; }
     else if (layout == ALLOYB_KV_Q8_PAGED) {
         if (!k1) return ALLOYB_E_NULL;

@@ -59,6 +59,7 @@ struct Params {
     int* status;
     AttnFuse fuse;           // valid when fused != 0: RoPE of q / new K and the K / V append happen in here
     int fused;
+    int v_half;              // fp16 cache: V starts 8 bytes past a 16-byte boundary
 };
 
 __device__ __forceinline__ uint32_t s32(const void* p) {
@@ -281,8 +282,14 @@ __global__ void __launch_bounds__(WARPS * 32) attn_mma_kernel(const Params P) {
                 const int64_t src = (head_row + min(t0 + tile * 16 + row, t1 - 1)) * D + c * 8;
                 const uint32_t at = dst + f16_piece(row, c);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at), "l"(static_cast<const __half*>(P.kv.k0) + src) : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + F16_TILE / 2), "l"(static_cast<const __half*>(P.kv.v0) + src)
-                             : "memory");
+                const __half* v = static_cast<const __half*>(P.kv.v0) + src;
+                if (!P.v_half) {
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + F16_TILE / 2), "l"(v) : "memory");
+                } else {                              // (a 16-byte copy would be misaligned, two of 8 bytes are not)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(at + F16_TILE / 2 + 8 * e), "l"(v + 4 * e) : "memory");
+                }
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -733,6 +740,7 @@ int launch_attn_mma(int layout, const void* q, int64_t q_bs, int64_t q_hs, int q
     P.B = B; P.H = H; P.KV_H = KV_H; P.G = H / KV_H;
     P.scale_log2 = scale_log2; P.splits = splits;
     P.part_o = part_o; P.part_lse = part_lse; P.counters = counters; P.status = status;
+    P.v_half = layout == ALLOYB_KV_F16 && reinterpret_cast<uintptr_t>(kv.v0) % 16 != 0;
     const dim3 grid(splits, KV_H, B);
     constexpr int F16_RING = am::WARPS * am::F16_SLOTS * am::F16_TILE;
     if (layout == ALLOYB_KV_F16) {

@@ -205,6 +205,21 @@ def test_kv_format_and_page_pool_host_logic():
         small.reserve(0, 48)
 
 
+def test_misaligned_f16_caches_are_refused_before_a_launch():
+    """Decode attention over an fp16 cache reads K 16 bytes at a time and, at head_dim 128, V at least 8: a cache that starts
+    elsewhere is an alignment error of the host's checks.  (No address here is ever touched.)"""
+    lib = _lib.load()
+    ok = 1 << 20
+    for d, k_off, v_off in ((128, 8, 0), (128, 2, 0), (128, 0, 4), (128, 0, 2), (64, 8, 0), (256, 0, 1)):
+        need = lib.alloyb_attn_workspace_bytes(1, 4, d)
+        kv_args = (0, ok, 4 * d, d)
+        caches = (ok + k_off, None, ok + v_off, None, ok, ok, d, d, ok, 1)
+        rc = lib.alloyb_attn_decode(*kv_args, _lib.F16, *caches, ok, 1, 4, 2, d, 32, 0, -1.0, 1, ok, need, None)
+        assert rc == -2, (d, k_off, v_off, rc)
+        rc = lib.alloyb_attn_decode_rope(*kv_args, *caches, ok, ok, 1, 4, 2, d, 32, 0, -1.0, ok, need, None)
+        assert rc == -2, (d, k_off, v_off, rc)
+
+
 def test_ops_import_without_a_cuda_build_of_torch():
     """A torch build without CUDA has no raw-stream query: the module still imports there and its Meta kernels work."""
     code = ("import torch\n"

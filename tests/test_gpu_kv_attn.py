@@ -442,3 +442,28 @@ def test_attention_f16_tiles_through_the_ring(b, kv_h, group, pos):
     s = q.double().unflatten(1, (kv_h, group)) @ k.double().unsqueeze(2).transpose(-1, -2) / np.sqrt(d)
     ref = (s.softmax(-1) @ v.double().unsqueeze(2)).flatten(1, 2)
     assert_close(to_np(out), ref.cpu().numpy(), torch.float16, f"f16 ring {b} {pos}")
+
+
+@pytest.mark.parametrize("b,kv_h,group,pos", [(2, 2, 4, 15), (1, 8, 4, 700), (3, 1, 7, 64)])
+def test_attention_f16_v_cache_eight_bytes_off(b, kv_h, group, pos):
+    """A V cache that starts 8 bytes past a 16-byte boundary: the same bits as an aligned one, by the op (append included)
+    and by the one-launch step."""
+    gen = torch.Generator(device=DEV).manual_seed(pos)
+    h, d, s_max = kv_h * group, 128, pos + 24
+    q, nk, nv = (torch.randn((b, n, d), device=DEV, generator=gen).half() for n in (h, kv_h, kv_h))
+    base = [torch.randn((b, kv_h, s_max, d), device=DEV, generator=gen).half() for _ in range(2)]
+    inv = (1.0 / (500000.0 ** (torch.arange(0, d, 2, dtype=torch.float32) / d))).to(DEV)
+    p = torch.tensor([pos], dtype=torch.int32, device=DEV)
+
+    def caches(shift):
+        v = torch.zeros(base[1].numel() + 16, dtype=torch.float16, device=DEV)[shift:shift + base[1].numel()].view(base[1].shape)
+        assert v.data_ptr() % 16 == 2 * shift
+        return base[0].clone(), v.copy_(base[1])
+
+    got = []
+    for shift in (0, 4):
+        a, f = caches(shift), caches(shift)
+        got.append((torch.ops.alloy.attention_cache(q.unsqueeze(2), nk.unsqueeze(2), nv.unsqueeze(2), p, *a, -1.0), *a,
+                    ops.rope_attention_decode(q, nk, nv, p, inv, k_cache=f[0], v_cache=f[1]), *f))
+    for x, y in zip(*got):
+        assert torch.equal(x, y)
