@@ -220,13 +220,14 @@ def linear_multi(x: torch.Tensor, specs: Sequence[tuple[str, torch.Tensor, torch
     if m == 0:
         return [x.new_empty((0, w.shape[0])) for _, w, _ in specs]
     descs = (Weight * len(specs))()
-    outs = []
+    outs, keep = [], []
     for i, (name, w, s) in enumerate(specs):
         fmt = _FORMATS[name]
         if _k_of(fmt, w) != k:
             raise ValueError("matrices must share K")
         y = torch.empty((m, w.shape[0]), dtype=x.dtype, device=x.device)
         w, pitch = _pitched(w)
+        keep.append(w)                  # a copy must outlive the launch's enqueueing, or the next matrix's takes its place
         descs[i] = Weight(fmt, w.shape[0], w.data_ptr(), s.data_ptr() if s is not None else None, pitch,
                           y.data_ptr(), 0)
         outs.append(y)

@@ -415,3 +415,36 @@ def test_q8_0_one_token(n, k, dt):
         y = torch.ops.alloy.linear_residual(xd, w[0], w[1], res, "q8_0")
         plain = torch.ops.alloy.gguf_q8_0_mm(xd, *w[:2])
         assert torch.equal(y, (res.float() + plain.float()).to(dt))
+
+
+@pytest.mark.parametrize("m", [1, 8, 24, 64])
+def test_packed_operands_that_are_copied_first(m):
+    """Views that no kernel reads directly (every other byte or column of a wider buffer, rewritten before each call) are
+    made contiguous on the stream: every call sees the copy of its own contents."""
+    rng = np.random.default_rng(m)
+    n, k = 640, 1024
+    x = torch.from_numpy((synth.activations(rng, m, k, np.float32) * 2 / np.sqrt(k)).astype(np.float16)).to(DEV)
+    q4 = [_dev(synth.q4k_blocks(rng, n, k)) for _ in range(6)]
+    q8 = [[_dev(a) for a in O.split_q8_0(synth.q8_0_wire(rng, n, k))] for _ in range(6)]
+
+    def spread(t):
+        return torch.empty((*t.shape[:-1], 2 * t.shape[-1]), dtype=t.dtype, device=DEV)[..., ::2]
+
+    views4, views8 = [spread(t) for t in q4[:2]], [spread(t) for t in (*q8[0], *q8[1])]
+    ops4 = (lambda a, b: [torch.ops.alloy.gguf_q4_k_silu(x, a, b)], lambda a, b: [torch.ops.alloy.gguf_q4_k_gelu(x, a, b)],
+            lambda a, b: [torch.ops.alloy.gguf_q4_k_mm(x, a)], lambda a, b: ops.linear_multi(x, [("q4_k", a, None), ("q4_k", b, None)]))
+    ops8 = (lambda *w: [torch.ops.alloy.gguf_q8_0_silu(x, *w)], lambda *w: [torch.ops.alloy.gguf_q8_0_mm(x, *w[:2])])
+    want, got = [], []
+    for i in range(0, 6, 2):
+        want += [y for op in ops4 for y in op(q4[i], q4[i + 1])] + [y for op in ops8 for y in op(*q8[i], *q8[i + 1])]
+    torch.cuda.synchronize()
+    for i in range(0, 6, 2):
+        for op in ops4:
+            for v, t in zip(views4, q4[i:i + 2]):
+                v.copy_(t)
+            got += op(*views4)
+        for op in ops8:
+            for v, t in zip(views8, (*q8[i], *q8[i + 1])):
+                v.copy_(t)
+            got += op(*views8)
+    assert len(want) == len(got) and all(torch.equal(a, b) for a, b in zip(want, got))
