@@ -14,6 +14,7 @@ LIB_PATH = _HERE / "liballoy_b200.so"
 
 F16, BF16, F32 = 0, 1, 2
 Q4_K, Q6_K, Q8_0 = 0, 1, 2
+CONST = 0x100          # OR-ed into the weight format of a linear call, see the header
 ACT_SILU, ACT_GELU_TANH = 0, 1
 KV_F16, KV_Q8_SPLIT, KV_Q8_PAGED = 0, 1, 2
 

@@ -109,7 +109,8 @@ static int validate_segs(const alloyb_weight* w, int n_w, int K, RowSegs& out) {
         if (!a.data || !a.y) return ALLOYB_E_NULL;
         if (a.N <= 0) return ALLOYB_E_SHAPE;
         int64_t dense;
-        switch (a.format) {
+        const int format = a.format & ~ALLOYB_CONST;
+        switch (format) {
             case ALLOYB_Q4_K:
                 if (K % QK_K) return ALLOYB_E_SHAPE;
                 dense = static_cast<int64_t>(K / QK_K) * Q4K_BYTES;
@@ -127,13 +128,14 @@ static int validate_segs(const alloyb_weight* w, int n_w, int K, RowSegs& out) {
                 return ALLOYB_E_SHAPE;
         }
         WeightSeg& s = out.seg[i];
-        s.format = a.format;
+        s.format = format;
+        s.constant = (a.format & ALLOYB_CONST) != 0;
         s.N = a.N;
         s.data = a.data;
         s.scales = a.scales;
         s.row_bytes = a.row_bytes ? a.row_bytes : dense;
         if (s.row_bytes < dense) return ALLOYB_E_SHAPE;
-        const int need = (a.format == ALLOYB_Q6_K) ? 2 : 4;
+        const int need = (format == ALLOYB_Q6_K) ? 2 : 4;
         if ((reinterpret_cast<uintptr_t>(a.data) % need) || (s.row_bytes % need)) return ALLOYB_E_ALIGN;
         s.y = a.y;
         s.ldy = a.ldy ? a.ldy : a.N;
@@ -170,7 +172,7 @@ static int linear_few_tokens(const void* x, int M, int K, int dtype, const RowSe
             bool taken = true;
             for (int i = 0; i < segs.n_seg && taken; ++i) {
                 const WeightSeg& sg = segs.seg[i];
-                rc = try_q8_gemv(x, M, K, dtype, sg.data, sg.scales, nullptr, nullptr, sg.y, sg.N, sg.ldy, residual, false, 0, st);
+                rc = try_q8_gemv(x, M, K, dtype, sg.data, sg.scales, nullptr, nullptr, sg.y, sg.N, sg.ldy, residual, false, 0, sg.constant, st);
                 if (rc == ALLOYB_NOT_TAKEN) taken = false;          // only possible for the first matrix (shape-wide reasons)
                 else if (rc != ALLOYB_OK) return rc;
             }
@@ -265,6 +267,8 @@ extern "C" int alloyb_gated_linear(const void* x, const void* gate, const void* 
     if (!x || !gate || !up || !y) return ALLOYB_E_NULL;
     if (M < 0 || N <= 0 || K <= 0) return ALLOYB_E_SHAPE;
     if (act != ALLOYB_ACT_SILU && act != ALLOYB_ACT_GELU_TANH) return ALLOYB_E_SHAPE;
+    const bool constant = (format & ALLOYB_CONST) != 0;
+    format &= ~ALLOYB_CONST;
     int64_t row_bytes;
     if (format == ALLOYB_Q4_K) {
         if (K % QK_K) return ALLOYB_E_SHAPE;
@@ -287,14 +291,14 @@ extern "C" int alloyb_gated_linear(const void* x, const void* gate, const void* 
         if (rc != ALLOYB_NOT_TAKEN) return rc;
     }
     if (M >= GEMM_TC_MIN_M) {
-        const WeightSeg g = {format, N, gate, gate_scales, row_bytes, y, N};
+        const WeightSeg g = {format, N, gate, gate_scales, row_bytes, y, N, constant};
         rc = try_gemm_tc(x, M, K, dtype, g, nullptr, up, up_scales, act, st);
         if (rc != ALLOYB_NOT_TAKEN) return rc;
     }
     rc = try_gated_fast(x, gate, gate_scales, up, up_scales, y, M, N, K, format, act, dtype, st);
     if (rc != ALLOYB_NOT_TAKEN) return rc;
     if (format == ALLOYB_Q8_0) {
-        rc = try_q8_gemv(x, M, K, dtype, gate, gate_scales, up, up_scales, y, N, N, nullptr, true, act, st);
+        rc = try_q8_gemv(x, M, K, dtype, gate, gate_scales, up, up_scales, y, N, N, nullptr, true, act, constant, st);
         if (rc != ALLOYB_NOT_TAKEN) return rc;
     }
 
@@ -350,7 +354,7 @@ extern "C" int alloyb_gated_linear_normed(const void* x, const void* norm_weight
     if (M < 0 || N <= 0 || K <= 0) return ALLOYB_E_SHAPE;
     if (act != ALLOYB_ACT_SILU && act != ALLOYB_ACT_GELU_TANH) return ALLOYB_E_SHAPE;
     if (M == 0) return ALLOYB_OK;
-    if (format == ALLOYB_Q4_K && K % QK_K == 0 && M == 1) {
+    if ((format & ~ALLOYB_CONST) == ALLOYB_Q4_K && K % QK_K == 0 && M == 1) {
         const int64_t rb = static_cast<int64_t>(K / QK_K) * Q4K_BYTES;
         const WeightSeg pair[2] = {{ALLOYB_Q4_K, N, gate, nullptr, rb, y, N}, {ALLOYB_Q4_K, N, up, nullptr, rb, y, N}};
         const int rc = try_gemv_stream(x, M, K, dtype, pair, 2, true, act, nullptr, norm_weight, eps, as_stream(stream), nullptr);

@@ -14,6 +14,7 @@ struct WeightSeg {
     int64_t row_bytes;
     void* y;
     int64_t ldy;
+    bool constant = false;             // ALLOYB_CONST: rows and scales may be requested before the launch before is over
 };
 
 // Tensor-core GEMV family / tcgen05 GEMM.  Return ALLOYB_NOT_TAKEN when the
@@ -48,7 +49,7 @@ int attn_prefill_device_error(int clear);
 
 // Q8_0 streaming GEMV (1..63 tokens, four per pass), plain (w1 == nullptr) or gate/up fused.
 int try_q8_gemv(const void* x, int M, int K, int dtype, const void* w0, const void* s0, const void* w1, const void* s1,
-                void* y, int N, int64_t ldy, const void* residual, bool gated, int act, cudaStream_t st);
+                void* y, int N, int64_t ldy, const void* residual, bool gated, int act, bool constant, cudaStream_t st);
 
 // tcgen05 dequant-GEMM for prefill-sized M (one matrix).
 // Fewer tokens go to the GEMV family: the tcgen05 kernel decodes every weight on the CUDA cores at about

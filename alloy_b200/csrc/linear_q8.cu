@@ -50,6 +50,7 @@ struct Params {
     int64_t ldy;
     const void* residual;            // plain only
     int act;
+    int constant;                    // codes and scales do not depend on earlier launches
 };
 
 // MTOK: tokens per pass (1: the decode case, light enough on registers for two CTAs per SM; 4)
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q8_gemv_one_kernel(const Params
                 o.s[a * R + r] = __ldg(P.s[a] + row * nblk + k / Q8_BLOCK);
             }
     };
-    // weights do not depend on the previous kernel
+    if (!P.constant) pdl_wait();                                  // a launch before this one may have written codes or scales
     Step even, odd;
     if (u0 < u1 && mine > 0) load(u0, 0, even);
     pdl_wait();
@@ -383,7 +384,7 @@ static int launch(const Params& P, cudaStream_t st) {
 // M tokens against one or two (gate/up) Q8_0 matrices; NOT_TAKEN when the shape or alignment is
 // outside the kernel (the row kernels then serve it).  More than four tokens run as passes of four.
 int try_q8_gemv(const void* x, int M, int K, int dtype, const void* w0, const void* s0, const void* w1, const void* s1,
-                void* y, int N, int64_t ldy, const void* residual, bool gated, int act, cudaStream_t st) {
+                void* y, int N, int64_t ldy, const void* residual, bool gated, int act, bool constant, cudaStream_t st) {
     if (M < 1 || M >= 64 || K % 512 || N < 1) return ALLOYB_NOT_TAKEN;
     const size_t esz = dtype == ALLOYB_F32 ? 4 : 2;
     if (static_cast<size_t>(q8::MT) * K * esz > 190 * 1024) return ALLOYB_NOT_TAKEN;
@@ -403,6 +404,7 @@ int try_q8_gemv(const void* x, int M, int K, int dtype, const void* w0, const vo
         P.ldy = ldy;
         P.residual = residual ? static_cast<const uint8_t*>(residual) + static_cast<size_t>(m0) * ldy * esz : nullptr;
         P.act = act;
+        P.constant = constant ? 1 : 0;
         int rc;
         if (dtype == ALLOYB_F16) rc = gated ? q8::launch<__half, true>(P, st) : q8::launch<__half, false>(P, st);
         else if (dtype == ALLOYB_BF16) rc = gated ? q8::launch<__nv_bfloat16, true>(P, st) : q8::launch<__nv_bfloat16, false>(P, st);

@@ -20,7 +20,7 @@ from dataclasses import dataclass
 
 import torch
 
-from . import ops, synth, tp
+from . import _lib, ops, synth, tp
 
 
 @dataclass(frozen=True)
@@ -77,7 +77,6 @@ class _FusedStep:
     def __init__(self, dec: "QuantLlamaDecoder") -> None:
         import ctypes as C
 
-        from . import _lib
         from ._lib import DecoderDesc, DecoderLayer, Matrix
 
         s = dec.shape
@@ -122,7 +121,6 @@ class _FusedStep:
         self.phases = int(L.alloyb_decoder_phases(self._handle))
 
     def step(self) -> None:
-        from . import _lib
         _lib.check(self._L.alloyb_decoder_step(self._handle, ops._stream()), "alloyb_decoder_step")
 
     def close(self) -> None:
@@ -325,7 +323,6 @@ class QuantLlamaDecoder:
     def device_error(self, clear: bool = True) -> int:
         """The library's sticky device error word (non-zero: a bounded wait ran out somewhere since
         it was last cleared, results since then are not to be trusted).  Synchronises the device."""
-        from . import _lib
         return int(_lib.load().alloyb_device_error(1 if clear else 0))
 
     def _step(self) -> None:
@@ -349,7 +346,7 @@ class QuantLlamaDecoder:
             # q/k (Q4_K) and v (Q6_K) of one token run as ONE streaming launch that also applies the input
             # RMSNorm (several tokens: the norm, then the projections)
             q, k, v = ops.linear_multi(h, [(lw.fmt["wq"], lw.wq, None), (lw.fmt["wk"], lw.wk, None),
-                                           (lw.fmt["wv"], lw.wv, None)], norm=(lw.norm_in, s.eps))
+                                           (lw.fmt["wv"], lw.wv, None)], norm=(lw.norm_in, s.eps), const=True)
             q3 = q.view(b, self.heads_l, s.head_dim)
             k3 = k.view(b, self.kv_heads_l, s.head_dim)
             v3 = v.view(b, self.kv_heads_l, s.head_dim)
@@ -372,20 +369,20 @@ class QuantLlamaDecoder:
                 a = a.transpose(1, 2)
             a2 = a.reshape(b, self.heads_l * s.head_dim)
             if self.tp_size == 1:
-                h = torch.ops.alloy.linear_residual(a2, lw.wo, None, h, lw.fmt["wo"])
+                h = ops._linear(a2, ops._FORMATS[lw.fmt["wo"]], [lw.wo], None, h, const=True)[0]
             else:
                 h = self._row_parallel(a2, lw.fmt["wo"], lw.wo, h)
             if lw.fmt["wg"] == "q4_k" and lw.fmt["wu"] == "q4_k":
-                act = ops.gated_normed(h, lw.norm_post, s.eps, lw.wg, lw.wu)
+                act = ops.gated_normed(h, lw.norm_post, s.eps, lw.wg, lw.wu, const=True)
             else:
                 gate, up = ops.linear_multi(h, [(lw.fmt["wg"], lw.wg, None), (lw.fmt["wu"], lw.wu, None)],
-                                            norm=(lw.norm_post, s.eps))
+                                            norm=(lw.norm_post, s.eps), const=True)
                 act = ops.silu_mul(gate, up)
             if self.tp_size == 1:
-                h = torch.ops.alloy.linear_residual(act, lw.wd, None, h, lw.fmt["wd"])
+                h = ops._linear(act, ops._FORMATS[lw.fmt["wd"]], [lw.wd], None, h, const=True)[0]
             else:
                 h = self._row_parallel(act, lw.fmt["wd"], lw.wd, h)
-        logits = ops.linear_multi(h, [(self.head_fmt, self.head, None)], norm=(self.norm_final, s.eps))[0]
+        logits = ops.linear_multi(h, [(self.head_fmt, self.head, None)], norm=(self.norm_final, s.eps), const=True)[0]
         if self.tp_size > 1 and not self.tp_dry:
             logits = tp.gather_columns(logits, self.pg)
         self.logits = logits
@@ -420,7 +417,7 @@ class QuantLlamaDecoder:
         for li, lw in enumerate(self.layers):
             xn = ops.rms_norm(x, lw.norm_in, s.eps)
             q, k, v = ops.linear_multi(xn, [(lw.fmt["wq"], lw.wq, None), (lw.fmt["wk"], lw.wk, None),
-                                            (lw.fmt["wv"], lw.wv, None)])
+                                            (lw.fmt["wv"], lw.wv, None)], const=True)
             q3 = q.view(m, self.heads_l, s.head_dim)
             k3 = k.view(m, self.kv_heads_l, s.head_dim)
             ops.rope_inplace(q3, k3, rows_pos, self.inv_freq)
@@ -435,21 +432,21 @@ class QuantLlamaDecoder:
                 a = torch.ops.alloy.attention_cache_q8_paged(q4, k4, v4, start_t, pool.page_table, pool.pool, -1.0, True)
             a2 = a.transpose(1, 2).reshape(m, self.heads_l * s.head_dim)
             if self.tp_size == 1:
-                x = torch.ops.alloy.linear_residual(a2, lw.wo, None, x, lw.fmt["wo"])
+                x = ops._linear(a2, ops._FORMATS[lw.fmt["wo"]], [lw.wo], None, x, const=True)[0]
             else:
                 x = self._row_parallel(a2, lw.fmt["wo"], lw.wo, x)
             xn = ops.rms_norm(x, lw.norm_post, s.eps)
             if lw.fmt["wg"] == "q4_k" and lw.fmt["wu"] == "q4_k":
-                act = torch.ops.alloy.gguf_q4_k_silu(xn, lw.wg, lw.wu)
+                act = ops._gated(xn, lw.wg, None, lw.wu, None, _lib.Q4_K, _lib.ACT_SILU, const=True)
             else:
-                gate, up = ops.linear_multi(xn, [(lw.fmt["wg"], lw.wg, None), (lw.fmt["wu"], lw.wu, None)])
+                gate, up = ops.linear_multi(xn, [(lw.fmt["wg"], lw.wg, None), (lw.fmt["wu"], lw.wu, None)], const=True)
                 act = ops.silu_mul(gate, up)
             if self.tp_size == 1:
-                x = torch.ops.alloy.linear_residual(act, lw.wd, None, x, lw.fmt["wd"])
+                x = ops._linear(act, ops._FORMATS[lw.fmt["wd"]], [lw.wd], None, x, const=True)[0]
             else:
                 x = self._row_parallel(act, lw.fmt["wd"], lw.wd, x)
         last = x.view(b, n, s.hidden)[:, -1].contiguous()
-        logits = ops.linear_multi(last, [(self.head_fmt, self.head, None)], norm=(self.norm_final, s.eps))[0]
+        logits = ops.linear_multi(last, [(self.head_fmt, self.head, None)], norm=(self.norm_final, s.eps), const=True)[0]
         if self.tp_size > 1 and not self.tp_dry:
             logits = tp.gather_columns(logits, self.pg)
         self.logits = logits

@@ -152,8 +152,9 @@ def _check_acts(x: torch.Tensor, k: int) -> torch.Tensor:
 
 
 def _linear(x: torch.Tensor, fmt: int, weights: Sequence[torch.Tensor],
-            scales: Sequence[torch.Tensor] | None, residual: torch.Tensor | None = None):
-    """One launch for ``len(weights)`` sibling matrices of one format."""
+            scales: Sequence[torch.Tensor] | None, residual: torch.Tensor | None = None, const: bool = False):
+    """One launch for ``len(weights)`` sibling matrices of one format.  ``const``: no earlier work of the stream writes
+    them (``ALLOYB_CONST``)."""
     if len(weights) == 0:
         return []
     k = _k_of(fmt, weights[0])
@@ -161,7 +162,7 @@ def _linear(x: torch.Tensor, fmt: int, weights: Sequence[torch.Tensor],
     m = x.shape[0]
     if m == 0:
         return [x.new_empty((0, w.shape[0])) for w in weights]
-    if len(weights) == 1 and fmt != _lib.Q8_0 and residual is None and weights[0].is_contiguous():
+    if len(weights) == 1 and fmt != _lib.Q8_0 and residual is None and not const and weights[0].is_contiguous():
         # one dense packed matrix, what a module's eager forward calls: the entry that takes plain arguments (4096 x 4096
         # for one token: the launch takes 5 us, descriptors and the general path cost the host 18 a call)
         w = weights[0]
@@ -191,7 +192,7 @@ def _linear(x: torch.Tensor, fmt: int, weights: Sequence[torch.Tensor],
             keep.append(s)
             s_ptr = s.data_ptr()
         keep.append(w)
-        descs[i] = Weight(fmt, w.shape[0], w.data_ptr(), s_ptr, pitch, y.data_ptr(), 0)
+        descs[i] = Weight(fmt | (_lib.CONST if const else 0), w.shape[0], w.data_ptr(), s_ptr, pitch, y.data_ptr(), 0)
         outs.append(y)
     r_ptr = None
     if residual is not None:
@@ -206,12 +207,13 @@ def _linear(x: torch.Tensor, fmt: int, weights: Sequence[torch.Tensor],
 
 
 def linear_multi(x: torch.Tensor, specs: Sequence[tuple[str, torch.Tensor, torch.Tensor | None]],
-                 norm: tuple[torch.Tensor, float] | None = None):
+                 norm: tuple[torch.Tensor, float] | None = None, const: bool = False):
     """Sibling projections of possibly different formats in ONE call.
 
     ``specs``: (format name, weight, scales-or-None) per matrix, all with the
     same K.  Used for q/k/v where v is Q6_K while q and k are Q4_K.
-    ``norm`` = (weight, eps): the projections see RMSNorm(x) (``alloyb_linear_normed``).
+    ``norm`` = (weight, eps): the projections see RMSNorm(x) (``alloyb_linear_normed``).  ``const``: no earlier work of the
+    stream writes the weights (``ALLOYB_CONST``).
     """
     fm0 = _FORMATS[specs[0][0]]
     k = _k_of(fm0, specs[0][1])
@@ -228,7 +230,7 @@ def linear_multi(x: torch.Tensor, specs: Sequence[tuple[str, torch.Tensor, torch
         y = torch.empty((m, w.shape[0]), dtype=x.dtype, device=x.device)
         w, pitch = _pitched(w)
         keep.append(w)                  # a copy must outlive the launch's enqueueing, or the next matrix's takes its place
-        descs[i] = Weight(fmt, w.shape[0], w.data_ptr(), s.data_ptr() if s is not None else None, pitch,
+        descs[i] = Weight(fmt | (_lib.CONST if const else 0), w.shape[0], w.data_ptr(), s.data_ptr() if s is not None else None, pitch,
                           y.data_ptr(), 0)
         outs.append(y)
     L = _lib.load()
@@ -270,8 +272,9 @@ def linear_allreduce(x: torch.Tensor, fmt_name: str, weight: torch.Tensor, resid
 
 
 def gated_normed(x: torch.Tensor, norm_weight: torch.Tensor, eps: float, gate: torch.Tensor, up: torch.Tensor,
-                 act: str = "silu") -> torch.Tensor:
-    """act(RMSNorm(x) G^T) * (RMSNorm(x) U^T) for Q4_K gate/up (``alloyb_gated_linear_normed``)."""
+                 act: str = "silu", const: bool = False) -> torch.Tensor:
+    """act(RMSNorm(x) G^T) * (RMSNorm(x) U^T) for Q4_K gate/up (``alloyb_gated_linear_normed``); ``const`` as in
+    ``linear_multi``."""
     k = _k_of(_lib.Q4_K, gate)
     x = _check_acts(x, k)
     y = torch.empty((x.shape[0], gate.shape[0]), dtype=x.dtype, device=x.device)
@@ -281,7 +284,7 @@ def gated_normed(x: torch.Tensor, norm_weight: torch.Tensor, eps: float, gate: t
     L = _lib.load()
     check(L.alloyb_gated_linear_normed(x.data_ptr(), norm_weight.data_ptr(), float(eps), scratch.data_ptr(),
                                        gate.data_ptr(), None, up.data_ptr(), None, y.data_ptr(), x.shape[0],
-                                       gate.shape[0], k, _lib.Q4_K,
+                                       gate.shape[0], k, _lib.Q4_K | (_lib.CONST if const else 0),
                                        _lib.ACT_SILU if act == "silu" else _lib.ACT_GELU_TANH, _dtype_code(x),
                                        _stream()), "alloyb_gated_linear_normed")
     return y
@@ -333,7 +336,7 @@ def _linear_residual(activations, weight, scales, residual, format):
     return _linear(activations, fmt, [weight], [scales] if scales is not None else None, residual)[0]
 
 
-def _gated(x, gate, gs, up, us, fmt, act):
+def _gated(x, gate, gs, up, us, fmt, act, const=False):
     k = _k_of(fmt, gate)
     if _k_of(fmt, up) != k or gate.shape[0] != up.shape[0]:
         raise ValueError("gate and up must have the same shape")
@@ -346,12 +349,12 @@ def _gated(x, gate, gs, up, us, fmt, act):
         # prefill: two single GEMMs + silu_mul, the split the reference measured faster than its
         # fused dual-accumulator kernel (packages/alloy-torch/src/alloy_torch/ops/linalg.py:774-780);
         # up to 128 tokens the tensor-core GEMM keeps both accumulators in tensor memory
-        g, u = _linear(x, fmt, [gate], None)[0], _linear(x, fmt, [up], None)[0]
+        g, u = _linear(x, fmt, [gate], None, const=const)[0], _linear(x, fmt, [up], None, const=const)[0]
         return silu_mul(g, u)
     L = _lib.load()
     check(L.alloyb_gated_linear(x.data_ptr(), gate.data_ptr(), gs.data_ptr() if gs is not None else None,
                                 up.data_ptr(), us.data_ptr() if us is not None else None,
-                                y.data_ptr(), x.shape[0], gate.shape[0], k, fmt, act,
+                                y.data_ptr(), x.shape[0], gate.shape[0], k, fmt | (_lib.CONST if const else 0), act,
                                 _dtype_code(x), _stream()), "alloyb_gated_linear")
     return y
 

@@ -28,6 +28,9 @@ extern "C" {
 enum { ALLOYB_F16 = 0, ALLOYB_BF16 = 1, ALLOYB_F32 = 2 };
 /* weight formats */
 enum { ALLOYB_Q4_K = 0, ALLOYB_Q6_K = 1, ALLOYB_Q8_0 = 2 };
+/* OR-ed into the weight format of a linear call: the packed rows and scales are constants, nothing the stream still has
+ * to run before the call writes them (see "quantised linear" below) */
+enum { ALLOYB_CONST = 0x100 };
 /* gate activation of the fused gate/up op */
 enum { ALLOYB_ACT_SILU = 0, ALLOYB_ACT_GELU_TANH = 1 };
 /* KV cache layouts */
@@ -87,8 +90,11 @@ int alloyb_dequant_q5_0(const void* qweight, const void* qhigh, const void* scal
  * reference's batched ops do by concatenating rows
  * (torch/ops/linalg.py:555-669, torch/custom_ops.py:50-52, :100-102, :106-108).
  *
- * Packed weights and their scales count as constants: the kernels request them while the kernel before them in
- * the stream is still draining (programmatic dependent launch); activations, residuals and outputs wait for it.
+ * Calls follow what earlier work of the stream wrote.  Where the format carries ALLOYB_CONST the kernels may request packed
+ * rows and scales while the kernel before them in the stream is still draining (programmatic dependent launch); without
+ * it they wait -- with one exception: below 28 tokens the fp16 / bf16 kernels for Q4_K and Q6_K do not, so a program
+ * that writes such rows on the stream puts one more operation (any plain kernel or a memset) between the write and
+ * the first of these calls.  Activations, residuals and outputs need nothing.
  *
  * M routing inside the library replaces torch/ops/linalg.py:462-497 (Q4_K),
  * :726-739 (Q6_K), :346-401 (Q8_0): small M runs the bandwidth-bound
@@ -98,7 +104,7 @@ int alloyb_dequant_q5_0(const void* qweight, const void* qhigh, const void* scal
  * dot_q4_k, :1949-1990 dot_q6_k and the load stage
  * metal/_compiler/msl/memory.py:441-879). */
 typedef struct alloyb_weight {
-    int format;              /* ALLOYB_Q4_K / Q6_K / Q8_0 */
+    int format;              /* ALLOYB_Q4_K / Q6_K / Q8_0, with ALLOYB_CONST where that holds */
     int N;                   /* output rows of this matrix */
     const void* data;        /* Q4_K/Q6_K: packed blocks (N, row_bytes); Q8_0: int8 (N,K) */
     const void* scales;      /* Q8_0: fp16 (N, K/32); else NULL */
@@ -134,7 +140,7 @@ int alloyb_q5_0_mm(const void* x, const void* qweight, const void* qhigh, const 
 /* y = act(x*G^T) * (x*U^T), one launch sharing the activation load
  * (torch/custom_ops.py:53-58 gguf_q4_k_silu/_gelu, :109-111 gguf_q8_0_silu;
  * kernels metal/std/quant.py:1458-1723, :358-695; policy torch/ops/linalg.py:758-802).
- * format is ALLOYB_Q4_K or ALLOYB_Q8_0 (scales NULL for Q4_K). */
+ * format is ALLOYB_Q4_K or ALLOYB_Q8_0 (scales NULL for Q4_K), with ALLOYB_CONST where that holds for both matrices. */
 int alloyb_gated_linear(const void* x, const void* gate, const void* gate_scales, const void* up,
                         const void* up_scales, void* y, int M, int N, int K, int format, int act,
                         int dtype, void* stream);

@@ -230,3 +230,21 @@ def test_ops_import_without_a_cuda_build_of_torch():
             "assert y.shape == (3, 40)\n")
     run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
     assert run.returncode == 0, run.stderr
+
+
+def test_weight_format_bits():
+    """ALLOYB_CONST is the only bit a format may carry; anything else is refused before a launch (none here touches memory)."""
+    lib = _lib.load()
+    ok = 1 << 20
+
+    def linear(fmt):
+        w = (_lib.Weight * 1)(_lib.Weight(fmt, 8, ok, ok, 0, ok, 0))
+        return lib.alloyb_linear(ok, 0, 512, _lib.F16, w, 1, None, None)
+
+    def gated(fmt):
+        return lib.alloyb_gated_linear(ok, ok, ok, ok, ok, ok, 0, 8, 512, fmt, _lib.ACT_SILU, _lib.F16, None)
+
+    for fmt in (_lib.Q4_K, _lib.Q6_K, _lib.Q8_0):
+        assert linear(fmt) == 0 and linear(fmt | _lib.CONST) == 0
+        assert linear(fmt | 0x200) == -1 and linear(fmt | 0x80) == -1
+        assert gated(fmt) == gated(fmt | _lib.CONST) == (-1 if fmt == _lib.Q6_K else 0) and gated(fmt | 0x200) == -1

@@ -225,3 +225,27 @@ def test_gemm_split_over_a_cluster(fmt, m, n, k, dt):
     torch.cuda.synchronize()
     assert all(torch.equal(y, o) for o in others)
     assert _lib.load().alloyb_device_error(0) == 0
+
+
+@pytest.mark.parametrize("m", [1, 20, 40, 200])
+def test_constant_weights_give_the_same_bits(m):
+    """ALLOYB_CONST says when packed rows may be requested, not what is computed: chains of dependent linears on one stream,
+    declared constant or not, agree bit for bit."""
+    rng = np.random.default_rng(m)
+    n = 1024
+    ws = [_dev((synth.q4k_blocks if i % 2 else synth.q6k_blocks)(rng, n, n)) for i in range(4)]
+    q8 = [_dev(a) for a in O.split_q8_0(synth.q8_0_wire(rng, n, 4096))]
+    x = _dev(synth.activations(rng, m, n, np.float32).astype(np.float16))
+    long = _dev(synth.activations(rng, m, 4096, np.float32).astype(np.float16))
+
+    def chain(const):
+        y, out = x, []
+        for _ in range(3):
+            for i, w in enumerate(ws):
+                y = ops.linear_multi(y, [("q4_k" if i % 2 else "q6_k", w, None)], const=const)[0]
+                y = (y.float() / y.float().abs().amax()).half()
+                out.append(y)
+        return out + ops.linear_multi(long, [("q8_0", *q8)], const=const)
+
+    assert all(torch.equal(a, b) for a, b in zip(chain(False), chain(True)))
+    assert _lib.load().alloyb_device_error(1) == 0
