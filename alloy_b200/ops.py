@@ -134,13 +134,23 @@ def _k_of(fmt: int, w: torch.Tensor) -> int:
     return w.shape[1] // bb * 256
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """A packed operand as a contiguous tensor.  Some kernels request packed rows while the launch before them is still
+    draining (``include/alloy_b200.h``), so a copy queued here gets one more operation behind it."""
+    if t.is_contiguous():
+        return t
+    t = t.contiguous()
+    torch.zeros(1, device=t.device)
+    return t
+
+
 def _pitched(w: torch.Tensor) -> tuple[torch.Tensor, int]:
     """A packed weight as (tensor, row pitch in bytes; 0 = dense).  Rows may be padded (a column
     shard whose row length is not a multiple of 16 bytes keeps a 16-byte pitch so that the
     tensor-core kernels can copy it); anything else is made contiguous."""
     if w.ndim == 2 and w.stride(1) == 1 and w.stride(0) >= w.shape[1] and w.element_size() == 1:
         return w, (0 if w.stride(0) == w.shape[1] else w.stride(0))
-    return w.contiguous(), 0
+    return _dense(w), 0
 
 
 def _check_acts(x: torch.Tensor, k: int) -> torch.Tensor:
@@ -188,7 +198,7 @@ def _linear(x: torch.Tensor, fmt: int, weights: Sequence[torch.Tensor],
             if s.dtype != torch.float16 or tuple(s.shape) != (w.shape[0], k // 32):
                 raise ValueError(f"q8_0 scales must be float16 {(w.shape[0], k // 32)}, "
                                  f"got {s.dtype} {tuple(s.shape)}")
-            s = s.contiguous()
+            s = _dense(s)
             keep.append(s)
             s_ptr = s.data_ptr()
         keep.append(w)
@@ -341,7 +351,7 @@ def _gated(x, gate, gs, up, us, fmt, act, const=False):
     if _k_of(fmt, up) != k or gate.shape[0] != up.shape[0]:
         raise ValueError("gate and up must have the same shape")
     x = _check_acts(x, k)
-    gate, up = gate.contiguous(), up.contiguous()
+    gate, up = _dense(gate), _dense(up)
     y = torch.empty((x.shape[0], gate.shape[0]), dtype=x.dtype, device=x.device)
     if x.shape[0] == 0:
         return y
@@ -371,8 +381,8 @@ def _q4k_gelu(activations, gate_blocks, up_blocks):
 
 @torch.library.impl(lib, "gguf_q8_0_silu", "CUDA")
 def _q8_silu(activations, gate_qweight, gate_scales, up_qweight, up_scales):
-    return _gated(activations, gate_qweight, gate_scales.contiguous(), up_qweight,
-                  up_scales.contiguous(), _lib.Q8_0, _lib.ACT_SILU)
+    return _gated(activations, gate_qweight, _dense(gate_scales), up_qweight,
+                  _dense(up_scales), _lib.Q8_0, _lib.ACT_SILU)
 
 
 # ------------------------------------------------------------------------------- Q5_0, routed experts
