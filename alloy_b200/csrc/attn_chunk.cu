@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
             const int64_t base = b * P.q_bs + static_cast<int64_t>(kvh * P.G + hgrp * 8 + hg) * P.q_hs +
                                  static_cast<int64_t>(tok0 + tl) * P.q_ts + d;
             if (q_vec) {
-                v = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(P.q) + base));
+                v = ld_after_wait(static_cast<const __half*>(P.q) + base);
             } else {
                 uint32_t* e = reinterpret_cast<uint32_t*>(&v);
 #pragma unroll

@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_mma_kernel(const Params P) {
         for (int kp = 0; kp < NKP; ++kp) {
             const int64_t base = b * P.q_bs + static_cast<int64_t>(kvh * G + g) * P.q_hs + 32 * kp + 8 * t;
             qraw[kp] = make_uint4(0u, 0u, 0u, 0u);
-            if (g < G) qraw[kp] = __ldg(reinterpret_cast<const uint4*>(static_cast<const __half*>(P.q) + base));
+            if (g < G) qraw[kp] = ld_after_wait(static_cast<const __half*>(P.q) + base);
         }
         if (P.fused) {
 #pragma unroll

@@ -205,8 +205,7 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(const Params P
         const int r = i >> 4, c = i & 15, tl = r >> P.gp_shift, hg = r & ((1 << P.gp_shift) - 1);
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (tok0 + tl < P.S && hg < heads_here)
-            v = __ldg(reinterpret_cast<const uint4*>(P.q + b * P.q_bs + static_cast<int64_t>(kvh * P.G + hgrp * 8 + hg) * P.q_hs +
-                                                     static_cast<int64_t>(tok0 + tl) * P.q_ts) + c);
+            v = ld_after_wait(P.q + b * P.q_bs + static_cast<int64_t>(kvh * P.G + hgrp * 8 + hg) * P.q_hs + static_cast<int64_t>(tok0 + tl) * P.q_ts + c * 8);
         *reinterpret_cast<uint4*>(smem + (r >> 7) * TILE + piece_at(r & 127, c)) = v;
     }
     fence_async();

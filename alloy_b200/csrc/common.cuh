@@ -81,6 +81,14 @@ __device__ __forceinline__ void pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Sixteen bytes that the launch before this one may have written, for use behind pdl_wait(): a load through the non-coherent
+// path (__ldg) is not bound to stay there, neither by the wait nor by its memory clobber.
+__device__ __forceinline__ uint4 ld_after_wait(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 // Launch with programmatic stream serialization allowed: the kernel may begin while its

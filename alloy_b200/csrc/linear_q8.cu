@@ -223,10 +223,10 @@ __global__ void __launch_bounds__(WARPS * 32, 2) q8_gemv_one_kernel(const Params
 #pragma unroll
     for (int sl = 0; sl < NS; ++sl) {
         const XT* xp = static_cast<const XT*>(P.x) + (warp + (sl < mine ? sl : 0) * WARPS) * SLICE + lane * 16;
-        XT v[16];
+        alignas(16) XT v[16];
 #pragma unroll
         for (int q = 0; q < 16 * static_cast<int>(sizeof(XT)) / 16; ++q)
-            reinterpret_cast<uint4*>(v)[q] = mine > 0 ? __ldg(reinterpret_cast<const uint4*>(xp) + q) : make_uint4(0u, 0u, 0u, 0u);
+            reinterpret_cast<uint4*>(v)[q] = mine > 0 ? ld_after_wait(reinterpret_cast<const uint4*>(xp) + q) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int e = 0; e < 8; ++e) x[sl][e] = pair(to_f32<XT>(v[2 * e]), to_f32<XT>(v[2 * e + 1]));
     }

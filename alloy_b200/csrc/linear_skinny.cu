@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(W * 32, MINB) linear_skinny_fixed_kernel(const
 #pragma unroll
             for (int p = 0; p < 2; ++p)
 #pragma unroll
-                for (int s = 0; s < 4; ++s) b[j][p][s][nt] = __ldg(reinterpret_cast<const uint4*>(xp + 32 * p + 8 * s));
+                for (int s = 0; s < 4; ++s) b[j][p][s][nt] = ld_after_wait(xp + 32 * p + 8 * s);
         }
         float sum[(NT + 1) / 2][4];
 #pragma unroll

@@ -81,3 +81,28 @@ def test_few_tokens_extreme_activations(scale):
     y = to_np(torch.ops.alloy.gguf_q4_k_mm(_dev(x), _dev(w))).astype(np.float64)
     bound = 2.0 ** -10 * np.abs(ref) + 2.0 ** -20 * (np.abs(x).astype(np.float64) @ np.abs(deq).T) + 2.0 ** -24
     assert keep.any() and (np.abs(y - ref)[keep] <= bound[keep]).all()
+
+
+@pytest.mark.parametrize("m", [1, 4, 16, 24])
+def test_tokens_that_the_launch_before_has_just_written(m):
+    """The normalised tokens come from the launch right before: read behind the wait, never ahead of it.  Calls queued back
+    to back, each on other tokens, against calls that are waited for one by one."""
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    n, k = 2 * torch.cuda.get_device_properties(0).multi_processor_count * 16 + 16, 4096
+    g, u = (synth.q4k_blocks_device(n, k, gen) for _ in range(2))
+    q8 = synth.q8_0_weight_device(n, k, gen)
+    w = torch.rand(k, device=DEV, generator=gen).half()
+    xs = [torch.randn((m, k), device=DEV, generator=gen).half() for _ in range(6)]
+
+    def calls(x):
+        return [ops.gated_normed(x, w, 1e-5, g, u), *ops.linear_multi(x, [("q4_k", g, None)], norm=(w, 1e-5)),
+                *ops.linear_multi(x, [("q8_0", *q8)], norm=(w, 1e-5))]
+
+    want = []
+    for x in xs:
+        xn = ops.rms_norm(x, w, 1e-5)
+        torch.cuda.synchronize()
+        want.append([torch.ops.alloy.gguf_q4_k_silu(xn, g, u), torch.ops.alloy.gguf_q4_k_mm(xn, g), torch.ops.alloy.gguf_q8_0_mm(xn, *q8)])
+        torch.cuda.synchronize()
+    for a, b in zip([calls(x) for x in xs], want):
+        assert all(torch.equal(p, q) for p, q in zip(a, b))
