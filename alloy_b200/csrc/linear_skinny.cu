@@ -588,8 +588,8 @@ __global__ void __launch_bounds__(WARPS * 32, 1) linear_skinny_kernel(const __gr
         for (int i = 0; i < 2048; ++i) __nanosleep(512);
 }
 
-// ---- up to sixteen tokens, rows of W * NSB super-blocks (K = 2048, 4096 or 8192): every warp keeps the token fragments of its
-// own NSB super-blocks in registers for the whole launch.
+// ---- up to sixteen tokens, rows of up to 32 super-blocks (9..16 tokens: 16): every one of a CTA's W warps keeps the token
+// fragments of its own NSB super-blocks in registers for the whole launch.
 //
 // In the kernel above the token path -- copies, waits, sums, once per super-block and warp -- took as long as the weights'
 // arithmetic at these sizes (gate/up 14336 x 4096, 8 tokens: 28 us, 14 of them without any weight arithmetic).  With the
@@ -601,6 +601,7 @@ template <int NSB> struct FixedGeom {
 };
 template <int NT, int W> struct FixedRed {
     static constexpr int WARP = 2 * 8 * NT * RED_PITCH, BYTES = 2 * W * WARP * 4;       // two tiles of a warp (floats); both buffers
+    static constexpr int BARS = (W * MAX_STAGES * 8 + 127) / 128 * 128;                 // (the rings behind it start on 128 bytes)
 };
 
 template <int NT, int W, int NSB, int MINB>
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(W * 32, MINB) linear_skinny_fixed_kernel(const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     float* red = reinterpret_cast<float*>(smem);
     const uint32_t bars = s32(smem) + FixedRed<NT, W>::BYTES + warp * MAX_STAGES * 8;
-    const uint32_t ring = s32(smem) + FixedRed<NT, W>::BYTES + W * MAX_STAGES * 8 + warp * P.stages * G::SLOT;
+    const uint32_t ring = s32(smem) + FixedRed<NT, W>::BYTES + FixedRed<NT, W>::BARS + warp * P.stages * G::SLOT;
     const int lo = static_cast<int>(static_cast<int64_t>(P.n_tiles) * blockIdx.x / gridDim.x);
     const int hi = static_cast<int>(static_cast<int64_t>(P.n_tiles) * (blockIdx.x + 1) / gridDim.x);
     if (lane == 0) {
@@ -644,7 +645,8 @@ __global__ void __launch_bounds__(W * 32, MINB) linear_skinny_fixed_kernel(const
     pdl_wait();      // activations (and the output buffer) belong to the previous kernel until here
 
     // ---- the tokens of this warp's super-blocks: fragments and split sums.  A column past the last token repeats the
-    // last one: columns do not mix, and it is never stored.
+    // last one: columns do not mix, and it is never stored.  A super-block past the row's end (an odd number of them, two per
+    // warp) is zero here and in the ring, whose tensor copies fill with zeros there.
     uint4 b[NSB][2][4][NT];
     uint2 sx[NSB][NT];
 #pragma unroll
@@ -655,7 +657,9 @@ __global__ void __launch_bounds__(W * 32, MINB) linear_skinny_fixed_kernel(const
 #pragma unroll
             for (int p = 0; p < 2; ++p)
 #pragma unroll
-                for (int s = 0; s < 4; ++s) b[j][p][s][nt] = ld_after_wait(xp + 32 * p + 8 * s);
+                for (int s = 0; s < 4; ++s)
+                    b[j][p][s][nt] = NSB == 1 || warp * NSB + j < P.nsb ? ld_after_wait(xp + 32 * p + 8 * s)
+                                                                        : make_uint4(0u, 0u, 0u, 0u);
         }
         float sum[(NT + 1) / 2][4];
 #pragma unroll
@@ -817,43 +821,87 @@ static int launch(const WeightSeg* seg, int n_mats, Params& P, cudaStream_t st) 
     return ALLOYB_OK;
 }
 
-template <int NT, int W, int NSB, int MINB>
+template <int NT, int W, int NSB>
 static int launch_fixed(const WeightSeg* seg, int n_mats, Params& P, cudaStream_t st) {
     using G = FixedGeom<NSB>;
     static bool configured[64] = {};
     static int sm_count[64] = {};
+    // CTAs per SM: as many as leave a thread the 128 registers (two token groups of two super-blocks: 255) that its fragments
+    // need.  28 KB are left to the first-level cache, through which the tokens come (K = 2048, 16 tokens, 4800 rows: 12.4 us
+    // without, 9.1 with), unless that leaves no ring.
+    constexpr int MINB = NT * NSB == 4 || W > 8 ? 1 : 16 / W;
+    constexpr int FIXED = 128 + FixedRed<NT, W>::BYTES + FixedRed<NT, W>::BARS, SLOTS = W * G::SLOT;
+    constexpr int FIT_CACHED = (200 * 1024 / MINB - 1024 - FIXED) / SLOTS, FIT_ALL = (228 * 1024 / MINB - 1024 - FIXED) / SLOTS;
+    constexpr int FIT = FIT_CACHED >= 2 ? FIT_CACHED : FIT_ALL, STAGES = FIT < MAX_STAGES ? FIT : MAX_STAGES, SMEM = FIXED + STAGES * SLOTS;
+    static_assert(FIT >= 2 && FixedRed<NT, W>::BYTES % 128 == 0 && G::SLOT % 256 == 0, "ring, and its 128-byte boundaries");
     auto kern = linear_skinny_fixed_kernel<NT, W, NSB, MINB>;
-    constexpr int SMEM_MAX = MINB == 1 ? 227 * 1024 : 113 * 1024, FIXED = 128 + FixedRed<NT, W>::BYTES + W * MAX_STAGES * 8;
-    constexpr int FIT = (SMEM_MAX - FIXED) / (W * G::SLOT);
-    static_assert(FIT >= 2, "ring");
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
         configured[dev] = true;
     }
-    // One tile per CTA does not pay for the tokens' way into the registers (4096 x 4096, 8 tokens: 8.4 us, the
-    // tokens-as-columns kernel of linear_mma.cu 5.5; 5120 x 4096, 16 tokens: 11.5 against 15.9).
-    if (P.n_tiles <= 2 * sm_count[dev]) return ALLOYB_NOT_TAKEN;
-    P.stages = FIT < MAX_STAGES ? FIT : MAX_STAGES;
+    // The tokens' way into the registers costs about three tiles' time, so whether it pays depends on the rounds of CTAs that the
+    // tokens-as-columns kernel of linear_mma.cu needs (16 rows each, a gate/up pair 16 of both; two per SM at once).  One
+    // round: that kernel (K = 4096, 8 tokens: 4096 rows 5.6 us, here 8.4; pair of 4000 7.9 / 11.3).  Two: this one (4800
+    // rows, 8 tokens 9.5 / 9.4, 16 tokens 15.4 / 11.8), except from five to eight tokens in middling rows where the second
+    // round is more than half full (8192 rows, 8 tokens: K = 2048 7.5 / 6.6, 4096 11.1 / 11.3, 6144 14.9 / 15.9, 8192 18.9 /
+    // 17.5).  More: this one (14336 rows, K = 3072: 8 tokens 18.4 / 15.2, 16 tokens 29.9 / 16.9).
+    const int sms = sm_count[dev], others = P.gated ? (P.seg[0].n_rows + 15) / 16 : P.n_tiles;
+    if (others <= 2 * sms) return ALLOYB_NOT_TAKEN;
+    if (P.M > 4 && P.M <= 8 && P.nsb > 8 && P.nsb < 28 && others > 3 * sms && others <= 4 * sms) return ALLOYB_NOT_TAKEN;
+    // (seven warps with two token groups each spill: 8192 rows, K = 1792, 16 tokens 10.6 / 11.9, 14336 rows 33.6 / 21.2)
+    if (NT == 2 && P.nsb == 7 && others <= 4 * sms) return ALLOYB_NOT_TAKEN;
+    P.stages = STAGES;
     Maps maps = {};
-    for (int i = 0; i < n_mats; ++i)
-        if (!map2d(&maps.one[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, seg[i].data, seg[i].row_bytes / 4, seg[i].N, seg[i].row_bytes, G::PITCH / 4,
-                   P.gated ? 8 : 16, CU_TENSOR_MAP_SWIZZLE_NONE)) {
+    for (int i = 0; i < n_mats; ++i)             // (the row's words only: what pads its pitch reads as zero)
+        if (!map2d(&maps.one[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, seg[i].data, static_cast<uint64_t>(P.nsb) * (Q4K_BYTES / 4), seg[i].N,
+                   seg[i].row_bytes, G::PITCH / 4, P.gated ? 8 : 16, CU_TENSOR_MAP_SWIZZLE_NONE)) {
             set_cuda_error(cudaErrorInvalidValue);
             return ALLOYB_E_CUDA;
         }
-    const int most = MINB * sm_count[dev], grid = P.n_tiles < most ? P.n_tiles : most;
-    const cudaError_t e = launch_pdl(kern, dim3(grid), dim3(W * 32), FIXED + W * P.stages * G::SLOT, st, maps, P);
+    const int most = MINB * sms, grid = P.n_tiles < most ? P.n_tiles : most;
+    const cudaError_t e = launch_pdl(kern, dim3(grid), dim3(W * 32), SMEM, st, maps, P);
     if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
     return ALLOYB_OK;
+}
+// One super-block per warp up to eight of them, two from there on.
+template <int NT>
+static int launch_fixed_rows(const WeightSeg* seg, int n_mats, Params& P, cudaStream_t st) {
+    switch (P.nsb <= 8 ? P.nsb : 100 + (P.nsb + 1) / 2) {
+        case 1: return launch_fixed<NT, 1, 1>(seg, n_mats, P, st);
+        case 2: return launch_fixed<NT, 2, 1>(seg, n_mats, P, st);
+        case 3: return launch_fixed<NT, 3, 1>(seg, n_mats, P, st);
+        case 4: return launch_fixed<NT, 4, 1>(seg, n_mats, P, st);
+        case 5: return launch_fixed<NT, 5, 1>(seg, n_mats, P, st);
+        case 6: return launch_fixed<NT, 6, 1>(seg, n_mats, P, st);
+        case 7: return launch_fixed<NT, 7, 1>(seg, n_mats, P, st);
+        case 8: return launch_fixed<NT, 8, 1>(seg, n_mats, P, st);
+        case 105: return launch_fixed<NT, 5, 2>(seg, n_mats, P, st);
+        case 106: return launch_fixed<NT, 6, 2>(seg, n_mats, P, st);
+        case 107: return launch_fixed<NT, 7, 2>(seg, n_mats, P, st);
+        case 108: return launch_fixed<NT, 8, 2>(seg, n_mats, P, st);
+    }
+    if constexpr (NT == 1) {                     // (two token groups: the registers hold no more than that)
+        switch ((P.nsb + 1) / 2) {
+            case 9: return launch_fixed<1, 9, 2>(seg, n_mats, P, st);
+            case 10: return launch_fixed<1, 10, 2>(seg, n_mats, P, st);
+            case 11: return launch_fixed<1, 11, 2>(seg, n_mats, P, st);
+            case 12: return launch_fixed<1, 12, 2>(seg, n_mats, P, st);
+            case 13: return launch_fixed<1, 13, 2>(seg, n_mats, P, st);
+            case 14: return launch_fixed<1, 14, 2>(seg, n_mats, P, st);
+            case 15: return launch_fixed<1, 15, 2>(seg, n_mats, P, st);
+            case 16: return launch_fixed<1, 16, 2>(seg, n_mats, P, st);
+        }
+    }
+    return ALLOYB_NOT_TAKEN;
 }
 
 }  // namespace sk
 
-// 2..32 fp16 tokens against Q4_K / Q6_K matrices: up to MAX_SEGS row-stacked outputs, or a Q4_K gate/up pair with the
+// 2..SKINNY_MAX_M fp16 tokens against Q4_K / Q6_K matrices: up to MAX_SEGS row-stacked outputs, or a Q4_K gate/up pair with the
 // activation fused.  NOT_TAKEN for anything else.
 int try_linear_skinny(const void* x, int M, int K, int dtype, const WeightSeg* seg, int n_seg, bool gated, int act,
                       const void* residual, cudaStream_t st) {
@@ -888,15 +936,7 @@ int try_linear_skinny(const void* x, int M, int K, int dtype, const WeightSeg* s
     P.act = act;
     if (M <= 16) {
         if (any_q6) return ALLOYB_NOT_TAKEN;
-        if (M <= 8) {
-            if (nsb == 8) return launch_fixed<1, 8, 1, 2>(seg, n_seg, P, st);
-            if (nsb == 16) return launch_fixed<1, 8, 2, 2>(seg, n_seg, P, st);
-            if (nsb == 32) return launch_fixed<1, 16, 2, 1>(seg, n_seg, P, st);
-        } else {
-            if (nsb == 8) return launch_fixed<2, 8, 1, 2>(seg, n_seg, P, st);
-            if (nsb == 16) return launch_fixed<2, 8, 2, 1>(seg, n_seg, P, st);
-        }
-        return ALLOYB_NOT_TAKEN;
+        return M <= 8 ? launch_fixed_rows<1>(seg, n_seg, P, st) : launch_fixed_rows<2>(seg, n_seg, P, st);
     }
     if (M <= 24) return launch<3, 4>(seg, n_seg, P, st);
     return launch<4, 4>(seg, n_seg, P, st);
