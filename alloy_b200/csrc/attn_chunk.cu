@@ -28,7 +28,6 @@ namespace alloyb {
 namespace ac {
 
 constexpr int ROWS = 64;          // (token, head) rows per CTA
-constexpr int KT = 64;            // KV tokens per tile
 constexpr int WARPS = 4;
 constexpr float NEG_BIG = -1.0e30f;
 constexpr float NEG_LIVE = 0.5f * NEG_BIG;    // scores above it are real
@@ -131,8 +130,10 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     return v;
 }
 
-template <int LAYOUT, int D>
+// KT: KV tokens per tile.  64; at head_dim 256 also 32, with which two CTAs (of ~100 KB) fit an SM.
+template <int LAYOUT, int D, int KT>
 struct Smem {
+    static constexpr int PARTS = WARPS * 32 / KT;                           // q8_0: threads that expand a token's row
     static constexpr int PITCH = D + 8;                                     // halves
     static constexpr int TILE = KT * PITCH * 2;                             // an fp16 tile of K or V
     static constexpr bool RAW = LAYOUT != ALLOYB_KV_F16;
@@ -143,10 +144,10 @@ struct Smem {
     static constexpr int BYTES = Q + (TILES > ROWS * D * 4 ? TILES : ROWS * D * 4) + 2 * ROWS * 4;
 };
 
-// Request tile j0 (64 tokens) of K (which = 0) or V (1): fp16 rows into the tile itself, q8 bytes into the raw buffer.
-template <int LAYOUT, int D>
+// Request tile j0 (KT tokens) of K (which = 0) or V (1): fp16 rows into the tile itself, q8 bytes into the raw buffer.
+template <int LAYOUT, int D, int KT>
 __device__ __forceinline__ void request_tile(uint32_t dst, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
-    using M = Smem<LAYOUT, D>;
+    using M = Smem<LAYOUT, D, KT>;
     const int tid = threadIdx.x;
     if (LAYOUT == ALLOYB_KV_Q8_PAGED) {
         // whole pages: a head's slab of 16 rows is contiguous
@@ -184,31 +185,33 @@ __device__ __forceinline__ void request_tile(uint32_t dst, const Params& P, int 
 }
 
 // The split layout's scales of this thread's blocks (see expand_tile), loaded a tile ahead.
-template <int D>
+template <int LAYOUT, int D, int KT>
 struct Scales {
-    __half s[D / 64];
+    static constexpr int N = D / 32 / Smem<LAYOUT, D, KT>::PARTS;
+    __half s[N];
 };
-template <int LAYOUT, int D>
-__device__ __forceinline__ void load_scales(Scales<D>& o, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
+template <int LAYOUT, int D, int KT>
+__device__ __forceinline__ void load_scales(Scales<LAYOUT, D, KT>& o, const Params& P, int which, int b, int kvh, int j0, int n_kv) {
     if (LAYOUT != ALLOYB_KV_Q8_SPLIT) return;
-    constexpr int NB = D / 32;
-    const int tok = threadIdx.x >> 1, j = min(j0 + tok, n_kv - 1);
+    using M = Smem<LAYOUT, D, KT>;
+    constexpr int NB = D / 32, N = Scales<LAYOUT, D, KT>::N;
+    const int tok = threadIdx.x / M::PARTS, j = min(j0 + tok, n_kv - 1);
     const __half* src = static_cast<const __half*>(which ? P.kv.v1 : P.kv.k1) +
-                        ((static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max + j) * NB + (threadIdx.x & 1) * (NB / 2);
+                        ((static_cast<int64_t>(b) * P.KV_H + kvh) * P.kv.S_max + j) * NB + (threadIdx.x % M::PARTS) * N;
 #pragma unroll
-    for (int i = 0; i < NB / 2; ++i) o.s[i] = __ldg(src + i);
+    for (int i = 0; i < N; ++i) o.s[i] = __ldg(src + i);
 }
 
-// Raw q8_0 bytes of a tile -> fp16(code * scale): two threads per token, half of its 32-code blocks each; tokens at or past
+// Raw q8_0 bytes of a tile -> fp16(code * scale): PARTS threads per token, their shares of its 32-code blocks; tokens at or past
 // n_kv become zero rows (whatever their page holds).
-template <int LAYOUT, int D>
-__device__ __forceinline__ void expand_tile(__half* dst, uint32_t raw, const Scales<D>& sc, int j0, int n_kv) {
-    using M = Smem<LAYOUT, D>;
-    constexpr int NB = D / 32;
-    const int tok = threadIdx.x >> 1, b0 = (threadIdx.x & 1) * (NB / 2);
+template <int LAYOUT, int D, int KT>
+__device__ __forceinline__ void expand_tile(__half* dst, uint32_t raw, const Scales<LAYOUT, D, KT>& sc, int j0, int n_kv) {
+    using M = Smem<LAYOUT, D, KT>;
+    constexpr int N = Scales<LAYOUT, D, KT>::N;
+    const int tok = threadIdx.x / M::PARTS, b0 = (threadIdx.x % M::PARTS) * N;
     const bool live = j0 + tok < n_kv;
 #pragma unroll
-    for (int i = 0; i < NB / 2; ++i) {
+    for (int i = 0; i < N; ++i) {
         uint32_t w[8];
         __half s;
         if (LAYOUT == ALLOYB_KV_Q8_PAGED) {
@@ -236,9 +239,9 @@ __device__ __forceinline__ void expand_tile(__half* dst, uint32_t raw, const Sca
     }
 }
 
-template <int LAYOUT, int D>
+template <int LAYOUT, int D, int KT>
 __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) {
-    using M = Smem<LAYOUT, D>;
+    using M = Smem<LAYOUT, D, KT>;
     pdl_launch_dependents();
     constexpr int PITCH = M::PITCH;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -268,15 +271,15 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
 
     auto request = [&](int tile, int buf) {
         const uint32_t at = s32(tiles) + (M::RAW ? 2 * M::TILE + buf * 2 * M::RAW_TILE : buf * 2 * M::TILE);
-        request_tile<LAYOUT, D>(at, P, 0, b, kvh, tile * KT, n_kv);
-        request_tile<LAYOUT, D>(at + (M::RAW ? M::RAW_TILE : M::TILE), P, 1, b, kvh, tile * KT, n_kv);
+        request_tile<LAYOUT, D, KT>(at, P, 0, b, kvh, tile * KT, n_kv);
+        request_tile<LAYOUT, D, KT>(at + (M::RAW ? M::RAW_TILE : M::TILE), P, 1, b, kvh, tile * KT, n_kv);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    Scales<D> sk, sv;
+    Scales<LAYOUT, D, KT> sk, sv;
     if (tile0 < tile1) {
         request(tile0, 0);
-        load_scales<LAYOUT, D>(sk, P, 0, b, kvh, tile0 * KT, n_kv);
-        load_scales<LAYOUT, D>(sv, P, 1, b, kvh, tile0 * KT, n_kv);
+        load_scales<LAYOUT, D, KT>(sk, P, 0, b, kvh, tile0 * KT, n_kv);
+        load_scales<LAYOUT, D, KT>(sv, P, 1, b, kvh, tile0 * KT, n_kv);
     }
 
     // ---- Q rows -> shared memory (fp16); dead rows are zero
@@ -335,11 +338,11 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
         uint32_t k_tile = s32(tiles) + buf * 2 * M::TILE;
         if (M::RAW) {
             const uint32_t raw = s32(tiles) + 2 * M::TILE + buf * 2 * M::RAW_TILE;
-            expand_tile<LAYOUT, D>(reinterpret_cast<__half*>(tiles), raw, sk, j0, n_kv);
-            expand_tile<LAYOUT, D>(reinterpret_cast<__half*>(tiles + M::TILE), raw + M::RAW_TILE, sv, j0, n_kv);
+            expand_tile<LAYOUT, D, KT>(reinterpret_cast<__half*>(tiles), raw, sk, j0, n_kv);
+            expand_tile<LAYOUT, D, KT>(reinterpret_cast<__half*>(tiles + M::TILE), raw + M::RAW_TILE, sv, j0, n_kv);
             if (more) {
-                load_scales<LAYOUT, D>(sk, P, 0, b, kvh, j0 + KT, n_kv);
-                load_scales<LAYOUT, D>(sv, P, 1, b, kvh, j0 + KT, n_kv);
+                load_scales<LAYOUT, D, KT>(sk, P, 0, b, kvh, j0 + KT, n_kv);
+                load_scales<LAYOUT, D, KT>(sv, P, 1, b, kvh, j0 + KT, n_kv);
             }
             k_tile = s32(tiles);
             __syncthreads();
@@ -498,15 +501,11 @@ __global__ void __launch_bounds__(WARPS * 32) attn_chunk_kernel(const Params P) 
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// CTAs below which the key range is split over a cluster: two per SM are resident, and a short chunk's few CTAs each walk
-// the whole history (77 tokens behind 1500, 32/8 heads: 40 CTAs of 25 tiles, 162 us of which one CTA's chain was all).
-constexpr int MIN_CTAS = 2 * 148;
-
-template <int LAYOUT, int D>
+template <int LAYOUT, int D, int KT>
 static int launch_one(Params& P, cudaStream_t st) {
     static bool configured[64] = {};
-    auto kern = attn_chunk_kernel<LAYOUT, D>;
-    constexpr int SMEM = Smem<LAYOUT, D>::BYTES;
+    auto kern = attn_chunk_kernel<LAYOUT, D, KT>;
+    constexpr int SMEM = Smem<LAYOUT, D, KT>::BYTES;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!configured[dev]) {
@@ -515,10 +514,6 @@ static int launch_one(Params& P, cudaStream_t st) {
         configured[dev] = true;
     }
     const int TQ = ROWS / P.Gp;
-    const int64_t ctas = static_cast<int64_t>((P.S + TQ - 1) / TQ) * P.KV_H * P.HG * P.B;
-    // the history's length is known on the device only; the cache's bounds it (four tiles per CTA at least)
-    P.splits = 1;
-    while (P.splits < 8 && ctas * P.splits < MIN_CTAS && P.kv.S_max >= 2 * P.splits * 4 * KT) P.splits *= 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((P.S + TQ - 1) / TQ * P.splits, P.KV_H * P.HG, P.B);
     cfg.blockDim = dim3(WARPS * 32);
@@ -538,12 +533,32 @@ static int launch_one(Params& P, cudaStream_t st) {
     return check_launch();
 }
 
+// The key range is split over a cluster while there are fewer CTAs than two per SM and the cache (the history's length is
+// known on the device only) has four tiles for each: a short chunk's few CTAs otherwise walk the whole history one tile
+// after the other (77 tokens behind 1500, 32/8 heads: 40 CTAs of 25 tiles, 162 us of which one CTA's chain was all).
 template <int LAYOUT>
 static int launch_d(Params& P, int D, cudaStream_t st) {
+    static int sm_count[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (!sm_count[dev]) {
+        int sms = 0;
+        const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
+        sm_count[dev] = sms;
+    }
+    const int TQ = ROWS / P.Gp, sms = sm_count[dev];
+    const int64_t ctas = static_cast<int64_t>((P.S + TQ - 1) / TQ) * P.KV_H * P.HG * P.B;
+    P.splits = 1;
+    while (P.splits < 8 && ctas * P.splits < 2 * sms && P.kv.S_max >= 2 * P.splits * 4 * 64) P.splits *= 2;
     switch (D) {
-        case 64: return launch_one<LAYOUT, 64>(P, st);
-        case 128: return launch_one<LAYOUT, 128>(P, st);
-        case 256: return launch_one<LAYOUT, 256>(P, st);
+        case 64: return launch_one<LAYOUT, 64, 64>(P, st);
+        case 128: return launch_one<LAYOUT, 128, 64>(P, st);
+        case 256:
+            // one CTA per SM is enough: the longer tiles (300 tokens, fp16: 27 us, with the shorter ones 38); more CTAs: two
+            // per SM (512 tokens, fp16 / q8_0 / paged: 102 / 131 / 141 us with the longer tiles, 74 / 102 / 111)
+            if (20 * ctas * P.splits <= 21 * sms) return launch_one<LAYOUT, 256, 64>(P, st);
+            return launch_one<LAYOUT, 256, 32>(P, st);
         default: return ALLOYB_E_SHAPE;
     }
 }

@@ -186,7 +186,10 @@ def test_chunk_attention_errors():
 
 @pytest.mark.parametrize("layout,b,kv_h,group,d,start,chunk", [
     ("f16", 1, 2, 4, 128, 1900, 3), ("f16", 1, 1, 1, 64, 0, 2), ("q8", 2, 1, 7, 128, 700, 40), ("q8", 1, 3, 4, 64, 1000, 18),
-    ("paged", 1, 2, 4, 128, 1999, 17), ("paged", 1, 1, 8, 256, 515, 2)])
+    ("paged", 1, 2, 4, 128, 1999, 17), ("paged", 1, 1, 8, 256, 515, 2),
+    # head_dim 256 with more CTAs than SMs: tiles of 32 tokens, split over a cluster and not
+    ("f16", 1, 8, 4, 256, 100, 130), ("q8", 1, 8, 4, 256, 61, 130), ("paged", 1, 8, 4, 256, 700, 40),
+    ("f16", 1, 64, 1, 256, 33, 270), ("q8", 1, 64, 1, 256, 1, 270), ("paged", 1, 64, 1, 256, 95, 257)])
 def test_chunk_over_a_split_history(layout, b, kv_h, group, d, start, chunk):
     """Few rows: the key range is split over a cluster whose CTAs merge through distributed shared memory; some CTAs get
     no tile, or none that a row may see."""
