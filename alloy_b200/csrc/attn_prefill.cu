@@ -408,13 +408,11 @@ __global__ void __launch_bounds__(THREADS, 1) attn_prefill_kernel(const Params P
 
 }  // namespace ap
 
-// NOT_TAKEN unless: fp16 queries in 16-byte-aligned rows, head_dim 128, an fp16 cache, and at least MIN_CTAS tiles of 256
-// (token, head) rows.
+// NOT_TAKEN unless: fp16 queries in 16-byte-aligned rows, head_dim 128, an fp16 cache, and enough live (token, head) rows in
+// tiles of 256.
 int try_attn_prefill(const void* q, int64_t q_bs, int64_t q_hs, int64_t q_ts, int q_dtype, const KVPtrs& kv, const int32_t* start,
                      int start_count, void* out, int B, int H, int KV_H, int dim, int n_tokens, float scale_log2, int* status, cudaStream_t st) {
     using namespace ap;
-    // a CTA here does the work of four of attn_chunk.cu's at twice their rate per SM: worth it from two thirds of the SMs on
-    constexpr int MIN_CTAS = 96;
     if (q_dtype != ALLOYB_F16 || dim != D) return ALLOYB_NOT_TAKEN;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out) | (q_bs * 2) | (q_hs * 2) | (q_ts * 2)) & 15) return ALLOYB_NOT_TAKEN;
     Params P;
@@ -430,15 +428,25 @@ int try_attn_prefill(const void* q, int64_t q_bs, int64_t q_hs, int64_t q_ts, in
     P.scale_log2 = scale_log2;
     P.status = status;
     const int TQ = ROWS >> P.gp_shift, tiles = (n_tokens + TQ - 1) / TQ;
-    if (static_cast<int64_t>(tiles) * KV_H * P.HG * B < MIN_CTAS) return ALLOYB_NOT_TAKEN;
     static bool configured[64] = {};
+    static int sm_count[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaError_t e = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
         configured[dev] = true;
     }
+    // Worth it from a third of the SMs on (32/8 heads: 448 tokens, 56 CTAs, 25.5 us against 28.0 of attn_chunk.cu, behind 1000
+    // more 51 / 80; 256 tokens, 32 CTAs, 18.2 / 18.5 and 42 / 48), unless most rows are dead.  Two of attn_chunk.cu's tiles of
+    // 64 rows cost an SM about as much as one tile here, so a chunk that it covers with fewer than two per tile stays there
+    // (batch 32, 16 tokens behind 300: 25 us, here 38; 32 tokens: 47 / 43) -- but for a single round that fills most of the
+    // SMs, where that kernel has to split its keys for it (16 tokens: batch 16 behind 3000 91 us, here 85; batch 12 behind 300
+    // 22 / 21, behind 3000 80 / 81).
+    const int64_t ctas = static_cast<int64_t>(tiles) * KV_H * P.HG * B, sms = sm_count[dev];
+    const int small_tiles = (n_tokens + TQ / 4 - 1) / (TQ / 4);
+    if (small_tiles < 2 * tiles ? 8 * ctas < 5 * sms || ctas > sms : 3 * ctas < sms) return ALLOYB_NOT_TAKEN;
     const cudaError_t e = launch_pdl(attn_prefill_kernel, dim3(tiles, KV_H * P.HG, B), dim3(THREADS), SMEM, st, P);
     if (e != cudaSuccess) { set_cuda_error(e); return ALLOYB_E_CUDA; }
     return check_launch();

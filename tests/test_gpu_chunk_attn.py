@@ -234,23 +234,55 @@ def test_chunk_over_a_split_history(layout, b, kv_h, group, d, start, chunk):
     assert_close(to_np(out), ref, torch.float16, f"split history {layout}")
 
 
-@pytest.mark.parametrize("b,kv_h,group,start,chunk", [(1, 8, 4, 0, 800), (2, 8, 7, 130, 321), (1, 32, 1, 1, 700), (3, 4, 16, 300, 133),
-                                                      (1, 96, 2, 127, 129), (1, 96, 1, 2000, 2)])
-def test_long_chunk_on_the_tensor_cores(b, kv_h, group, start, chunk):
+def _chunk_ref(q, k, v, starts, scale):
+    """Causal attention in 64 bits: q (B, H, S, D), k and v (B, KV_H, N, D) with every row a sequence may see."""
+    group, chunk, n = q.shape[1] // k.shape[1], q.shape[2], k.shape[2]
+    s = q.double().unflatten(1, (-1, group)) @ k.double().unsqueeze(2).transpose(-1, -2) * scale
+    last = torch.as_tensor(starts, device=DEV).view(-1, 1) + torch.arange(chunk, device=DEV)
+    seen = torch.arange(n, device=DEV) <= last.unsqueeze(-1)
+    return (s.masked_fill(~seen.view(-1, 1, 1, chunk, n), -np.inf).softmax(-1) @ v.double().unsqueeze(2)).flatten(1, 2)
+
+
+@pytest.mark.parametrize("b,kv_h,group,start,chunk,scale", [
+    (1, 8, 4, 0, 800, -1.0), (2, 8, 7, 130, 321, -1.0), (1, 32, 1, 1, 700, 0.05), (3, 4, 16, 300, 133, -1.0),
+    (1, 96, 2, 127, 129, 0.2), (1, 96, 1, 2000, 256, -1.0), (1, 8, 4, 40, 420, -1.0), (16, 8, 4, 50, 3, -1.0)])
+def test_long_chunk_on_the_tensor_cores(b, kv_h, group, start, chunk, scale):
     """Enough rows for the tcgen05 kernel: tiles of 256 rows and 128 keys with ragged ends, padded head groups, scores that
-    make the maximum climb, and a cache whose unused rows hold NaN."""
+    make the maximum climb, a cache whose unused rows hold NaN, a scale of the caller's; q as the model code has it, a
+    transposed view of (B, S, H, D)."""
     gen = torch.Generator(device=DEV).manual_seed(b * 1000 + chunk)
     h, d, n, s_max = kv_h * group, 128, start + chunk, start + chunk + 150
     rows = [torch.randn((b, kv_h, n, d), device=DEV, generator=gen).half() for _ in range(2)]
     rows[0] *= torch.linspace(0.2, 6.0, n, device=DEV).half().view(n, 1)         # later keys score higher
-    q = torch.randn((b, h, chunk, d), device=DEV, generator=gen).half()
+    q = torch.randn((b, chunk, h, d), device=DEV, generator=gen).half().transpose(1, 2)
     caches = [torch.full((b, kv_h, s_max, d), float("nan"), dtype=torch.float16, device=DEV) for _ in range(2)]
     for c, r in zip(caches, rows):
         c[:, :, :start] = r[:, :, :start]
     new = [r[:, :, start:].transpose(1, 2).contiguous().transpose(1, 2) for r in rows]
-    out = torch.ops.alloy.attention_cache(q, *new, torch.tensor([start], device=DEV), *caches, -1.0)
-    s = q.double().unflatten(1, (kv_h, group)) @ rows[0].double().unsqueeze(2).transpose(-1, -2) / np.sqrt(d)
-    seen = torch.arange(n, device=DEV) <= start + torch.arange(chunk, device=DEV).unsqueeze(1)
-    ref = (s.masked_fill(~seen, -np.inf).softmax(-1) @ rows[1].double().unsqueeze(2)).flatten(1, 2)
+    pos = torch.tensor([start], device=DEV)
+    out = torch.ops.alloy.attention_cache(q, *new, pos, *caches, scale)
+    ref = _chunk_ref(q, *rows, [start], scale if scale > 0 else 1 / np.sqrt(d))
     assert_close(to_np(out), ref.cpu().numpy(), torch.float16, "long chunk")
+    assert torch.equal(torch.ops.alloy.attention_cache(q.contiguous(), *new, pos, *caches, scale), out)
     assert _lib.load().alloyb_device_error(1) == 0
+
+
+@pytest.mark.parametrize("kv_h,group,starts,chunk", [(8, 4, [0, 700, 127], 300), (16, 3, [1, 255, 30, 129], 129)])
+def test_long_chunk_with_a_start_per_sequence(kv_h, group, starts, chunk):
+    """The C entry with one start per sequence, the chunk's rows already in the fp16 cache."""
+    gen = torch.Generator(device=DEV).manual_seed(chunk)
+    b, h, d, s_max = len(starts), kv_h * group, 128, max(starts) + chunk + 40
+    k, v = (torch.randn((b, kv_h, s_max, d), device=DEV, generator=gen).half() for _ in range(2))
+    q = torch.randn((b, chunk, h, d), device=DEV, generator=gen).half().transpose(1, 2)
+    ref = _chunk_ref(q, k, v, starts, 1 / np.sqrt(d))
+    for i, s in enumerate(starts):
+        k[i, :, s + chunk:] = v[i, :, s + chunk:] = float("nan")
+    start = torch.tensor(starts, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = torch.empty((b, chunk, h, d), dtype=torch.float16, device=DEV)
+    L = _lib.load()
+    _lib.check(L.alloyb_attn_chunk(_lib.KV_F16, q.data_ptr(), q.stride(0), q.stride(1), q.stride(2), _lib.F16, k.data_ptr(), None,
+                                   v.data_ptr(), None, start.data_ptr(), b, out.data_ptr(), b, h, kv_h, d, chunk, s_max, 0, -1.0,
+                                   status.data_ptr(), torch.cuda.current_stream().cuda_stream), "attn_chunk")
+    assert_close(to_np(out), ref.transpose(1, 2).cpu().numpy(), torch.float16, "starts per sequence")
+    assert int(status.item()) == 0 and L.alloyb_device_error(1) == 0
