@@ -111,6 +111,8 @@ __global__ void rope_kernel(T* __restrict__ q, T* __restrict__ k, const int32_t*
 // of its heads (the kernel above spends its time in sincosf, D/2 of them per head) and a thread rotates eight pairs with
 // 16-byte loads and stores.  2048 tokens x 40 heads x 128: 31.9 -> 7.3 us.
 constexpr int ROPE_MAX_HALF = 256;
+constexpr int ROPE_ROWS_MIN_TOKENS = 72;
+constexpr int64_t ROPE_ROWS_MIN_PAIRS = 80 * 1024;
 template <typename T>
 __global__ void __launch_bounds__(256) rope_rows_kernel(T* __restrict__ q, T* __restrict__ k, const int32_t* __restrict__ pos, int pos_count,
                                                         const float* __restrict__ inv_freq, int H, int KV_H, int D) {
@@ -300,8 +302,10 @@ extern "C" int alloyb_rope_inplace(void* q, void* k, const int32_t* pos, int pos
     const int64_t total = static_cast<int64_t>(B) * (H + KV_H) * (D / 2);
     const int blocks = static_cast<int>((total + 255) / 256);
     cudaStream_t st = as_stream(stream);
-    // whole 16-byte pieces of a head's halves: the row kernel (measured, 2048 x 40 x 128 fp16: 31.9 us element by element)
-    if (dtype != ALLOYB_F32 && D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0) {
+    // whole 16-byte pieces of a head's halves: the row kernel, from as many tokens on as its CTAs (one per token) need to fill
+    // half the SMs (40 heads of 128: 16 tokens 2.1 us element by element, 2.8 by rows; 64 2.9 / 2.9; 128 3.4 / 3.0; 2048
+    // 28.5 / 7.3) and rows that are worth a CTA (10 heads: 96 tokens 2.2 / 2.35, 128 2.3 / 2.3, 400 3.1 / 2.4)
+    if (B >= ROPE_ROWS_MIN_TOKENS && total >= ROPE_ROWS_MIN_PAIRS && dtype != ALLOYB_F32 && D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0) {
         const cudaError_t e =
             dtype == ALLOYB_F16
                 ? launch_pdl(rope_rows_kernel<__half>, dim3(B), dim3(256), 0, st, static_cast<__half*>(q), static_cast<__half*>(k), pos, pos_count,

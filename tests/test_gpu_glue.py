@@ -69,11 +69,11 @@ def test_argmax_first_maximum(m, n, dt):
     assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("b,h,kvh,d,dt", [(1, 32, 8, 128, torch.float16), (70, 5, 1, 64, torch.bfloat16), (3, 2, 2, 256, torch.float16),
-                                          (2, 3, 1, 48, torch.float16)])
+@pytest.mark.parametrize("b,h,kvh,d,dt", [(110, 32, 8, 128, torch.float16), (300, 27, 1, 64, torch.bfloat16), (120, 16, 2, 256, torch.float16),
+                                          (300, 36, 1, 48, torch.float16), (1, 32, 8, 128, torch.float16)])
 def test_rope_rows_equal_the_scalar_kernel(b, h, kvh, d, dt):
-    """Aligned 16-bit rows take the kernel that rotates eight pairs per thread, unaligned ones go element by element:
-    bit for bit the same."""
+    """Aligned 16-bit rows take the kernel that rotates eight pairs per thread (many tokens: all cases but the last),
+    unaligned ones go element by element: bit for bit the same."""
     gen = torch.Generator().manual_seed(b)
     q, k = torch.randn((b, h, d), generator=gen).to(dt).to(DEV), torch.randn((b, kvh, d), generator=gen).to(dt).to(DEV)
     pos = torch.randint(0, 9000, (b,), generator=gen, dtype=torch.int32).to(DEV)
