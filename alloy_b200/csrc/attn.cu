@@ -422,8 +422,8 @@ static int attn_decode_run(int layout, const void* q, int64_t q_batch_stride, in
     P.part_o = reinterpret_cast<float*>(ws);
 
     // Split count: the (b, kv head) pairs times the splits run in waves of as many CTAs per SM as the
-    // layout's kernel keeps resident (registers: 2 for the fp16 cache, whose tiles are staged in registers,
-    // 3 for the split q8_0 cache, 4 for the paged pool); a split costs its tokens (whole 64-token passes of
+    // layout's kernel keeps resident (2 for the fp16 cache, by the shared memory of its tiles; by registers 3 for
+    // the split q8_0 cache and 4 for the paged pool); a split costs its tokens (whole 64-token passes of
     // the four warps) plus a fixed start-up and merge share, and every extra split lengthens the final
     // merge.  Take the cheapest.
     const int ctas = B * KV_H;

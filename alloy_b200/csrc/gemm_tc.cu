@@ -14,9 +14,8 @@
 //   * the packed-row warp (one lane) brings the 128 packed weight rows of a super-block (four K steps) in
 //     with ONE tensor copy over a byte view of the weight matrix (Q8_0: two swizzled copies of codes and
 //     one of scales), issued as soon as the slot's previous super-block is decoded;
-//   * the decode warps work in DG groups of four warps that take K steps round robin, so each group has
-//     DG step times for its chain of waits, loads and stores (DG = 2 under the 256-token tile, whose
-//     epilogue needs the registers; 4 otherwise, where decode alone bounds the kernel); a thread sits on the
+//   * the decode warps work in four groups of four warps, one for each K step of a super-block, so each group
+//     has four step times for its chain of waits, loads and stores; a thread sits on the
 //     tensor-memory lane of its weight row and decodes the row's 64 weights of the step to fp32 exactly
 //     as the block format defines them (Q4_K: d*sc*nib - dmin*m with ONE rounding; Q6_K: d*sc*(q-32),
 //     exact; Q8_0: scale*code, exact), rounds ONCE to the activation type and stores 32 packed columns.
@@ -71,22 +70,23 @@ static_assert(2 * Q8_STAGE <= PACK_BYTES && 5 * Q4_STAGE <= PACK_BYTES, "packed-
 // walks a box row by row, and several short boxes in flight finish sooner than one tall one.
 constexpr int PACK_BOXES = 4, PACK_BOX_ROWS = BN / PACK_BOXES;
 constexpr int DEC_GROUP = 128;          // one decode group: a thread per weight row
+constexpr int DEC_GROUPS = 4;           // one for each K step of a super-block
 constexpr int EPI_THREADS = 256;        // two per accumulator lane (half of the token columns each)
 constexpr uint32_t SPIN = 1u << 22;
 constexpr int GATED_MAX_BM = 128;       // tokens of a gate/up pair (two accumulators)
 constexpr int MAX_SPLITS = 8;           // K ranges of a tile = CTAs of a cluster
 
-template <int BM, int DG>
+template <int BM>
 struct Cfg {
     static constexpr int X_STAGE = BM * BK * 2;                 // one token tile
-    // Stages of tokens (shared memory) and decoded weights (tensor memory).  With DG decode groups on
-    // DG stages every group would wait for the MMAs of its own previous step before it may store the
+    // Stages of tokens (shared memory) and decoded weights (tensor memory).  With the four decode groups on
+    // four stages every group would wait for the MMAs of its own previous step before it may store the
     // next one; twice as many stages let it run a step ahead.
     static constexpr int STAGES = BM <= 128 ? 8 : 4;
     // Warps 0-3: token copies, MMA, packed-row copies, (narrow tiles) a second MMA issuer; then the decode groups, then
     // the epilogue, then further issuers.  Groups of four start at multiples of four: a warp's index modulo four is its
     // quarter of tensor memory, and register counts are set by such groups.
-    static constexpr int PACK_WARP = 2, DEC_WARP0 = 4, EPI_WARP0 = DEC_WARP0 + 4 * DG;
+    static constexpr int PACK_WARP = 2, DEC_WARP0 = 4, EPI_WARP0 = DEC_WARP0 + 4 * DEC_GROUPS;
     // The 256-token tile runs 28 warps at 72 registers a thread: the epilogue, which holds 128 results per thread, takes
     // over what the other roles can spare.  (56 x 128 + 56 x 512 + 112 x 256 = 72 x 896.)
     static constexpr bool SHARE_REGS = BM == 256;
@@ -367,15 +367,15 @@ struct StageGate {
 
 // Decode k-step `ks` (0..3) of one Q4_K super-block of this thread's row: 64 weights = the low
 // nibbles (sub-block 2*ks, k 0..31 -> columns 0..15) and the high nibbles (sub-block 2*ks + 1,
-// k 32..63 -> columns 16..31) of 32 quant bytes.  UPPER: ks >= 2 (sub-blocks 4-7, whose scales are put together from
-// two places) -- 0 or 1 where it is known at compile time, -1 where it is not.
-template <bool BF16, int UPPER>
+// k 32..63 -> columns 16..31) of 32 quant bytes.  (From ks = 2 on -- sub-blocks 4-7 -- the scales are put together from
+// two places.)
+template <bool BF16>
 __device__ __forceinline__ void decode_q4k(const uint8_t* blk, const uint4& hdr, int ks, uint32_t dst, StageGate& gate) {
     const uint4 q0 = lds_u128(blk + 16 + ks * 32), q1 = lds_u128(blk + 32 + ks * 32);
     const float d = half_bits_to_f32(hdr.x & 0xffffu), dmin = half_bits_to_f32(hdr.x >> 16);
     const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
     const uint64_t unbias = f2(-8388608.0f, -8388608.0f);
-    const bool upper = UPPER < 0 ? ks >= 2 : UPPER == 1;
+    const bool upper = ks >= 2;
     const uint32_t sc4 = upper ? (hdr.w & 0x0f0f0f0fu) | ((hdr.y >> 2) & 0x30303030u) : hdr.y & 0x3f3f3f3fu;
     const uint32_t mn4 = upper ? ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u) : hdr.z & 0x3f3f3f3fu;
     const uint32_t sel = 0x7540u | (2u * (ks & 1));
@@ -533,10 +533,10 @@ __device__ __forceinline__ void load_sum(uint32_t addr, uint32_t (&v)[8]) {
     }
 }
 
-template <bool BF16, int BM, int DG>
-__global__ void __launch_bounds__(Cfg<BM, DG>::THREADS, 1)
+template <bool BF16, int BM>
+__global__ void __launch_bounds__(Cfg<BM>::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
-    using C = Cfg<BM, DG>;
+    using C = Cfg<BM>;
     constexpr int X_STAGE = C::X_STAGE, STAGES = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -558,7 +558,7 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
         }
         for (int s = 0; s < PACK_MAX_STAGES; ++s) {
             bar_init(&bars->p_full[s], 1);
-            bar_init(&bars->p_empty[s], DG * DEC_GROUP);
+            bar_init(&bars->p_empty[s], DEC_GROUPS * DEC_GROUP);
         }
         bar_init(&bars->acc_full, C::NI);
         bar_init(&bars->acc_empty, EPI_THREADS);
@@ -699,15 +699,12 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
     } else if (warp < C::EPI_WARP0) {
         if (C::SHARE_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         // ------------------------------------------------ decode: thread = weight row = the tensor-memory
-        // lane this warp may access (its index modulo 4 picks the quarter); group g takes the k-steps whose
-        // running count is g modulo DG
+        // lane this warp may access (its index modulo 4 picks the quarter); group g takes k-step g
+        // of every super-block
         const int r = (warp & 3) * 32 + lane, g = (warp - C::DEC_WARP0) >> 2;
         const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + C::W_COL0;
-        // A super-block is four k-steps and DG divides four: group g has the steps g, g + DG, ... of every super-block,
-        // so that a step's place in the block is known at compile time (DG = 2: up to the group's parity) and the header
-        // is read once.  Ring positions are counted, not divided out.  (Steps dealt out one by one, with divisions by the
-        // run-time ring depth, and two groups under the 256-token tile: 14336 x 4096 at 2048 tokens 237 us, now 216; gate/up
-        // at 32 tokens 56, now 50.)
+        // (Steps dealt out one by one, with divisions by the run-time ring depth, and two groups under the 256-token
+        // tile: 14336 x 4096 at 2048 tokens 237 us, so 216; gate/up at 32 tokens 56, so 50.)
         auto decode_all = [&](auto format) {
             constexpr int FMT = decltype(format)::value;
             bool ok = true;
@@ -723,31 +720,25 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                     // (a gate/up pair walks K twice: the block's place in its row starts over)
                     const int k_sb = sb - im.sb0 * n_sub;
                     const uint32_t off6 = ((im.sb0 + (k_sb >= im.sb1 - im.sb0 ? k_sb - (im.sb1 - im.sb0) : k_sb)) * Q6K_BYTES) & 15;
-                    auto step = [&](auto index) {
-                        constexpr int J = decltype(index)::value;
-                        const int ks = g + DG * J;
-                        const uint32_t it = sbi * 4 + ks, s = it % STAGES;
-                        // the stage's previous use must be over before the first store to it, not before
-                        // the loads and the arithmetic: test now, and only wait (inside the decode, right
-                        // before its first tensor-memory store) if the test failed
-                        const uint32_t e_bar = s32(&bars->empty[s]), e_par = ((it / STAGES) - 1) & 1;
-                        const bool free_now = it < STAGES || bar_test_a(e_bar, e_par);
-                        if (ok) {
-                            const uint32_t dst = lane_base + s * W_COLS;
-                            StageGate gate{e_bar, e_par, free_now, true};
-                            // rows past N arrive as zeros from the tensor copy and decode to zeros
-                            if (FMT == ALLOYB_Q4_K) decode_q4k<BF16, DG == 2 ? J : -1>(row, hdr, ks, dst, gate);
-                            else if (FMT == ALLOYB_Q6_K) decode_q6k<BF16>(row + off6, ks, dst, gate);
-                            else decode_q8_0<BF16>(stg, ks, r, dst, gate);
-                            ok = gate.ok;
-                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                        }
-                        bar_arrive(&bars->full[s]);
-                    };
-                    step(std::integral_constant<int, 0>{});
-                    if (DG == 2) step(std::integral_constant<int, DG == 2 ? 1 : 0>{});
-                    // every decode thread releases the super-block once, after its last step of it
+                    const uint32_t it = sbi * 4 + g, s = it % STAGES;
+                    // the stage's previous use must be over before the first store to it, not before
+                    // the loads and the arithmetic: test now, and only wait (inside the decode, right
+                    // before its first tensor-memory store) if the test failed
+                    const uint32_t e_bar = s32(&bars->empty[s]), e_par = ((it / STAGES) - 1) & 1;
+                    const bool free_now = it < STAGES || bar_test_a(e_bar, e_par);
+                    if (ok) {
+                        const uint32_t dst = lane_base + s * W_COLS;
+                        StageGate gate{e_bar, e_par, free_now, true};
+                        // rows past N arrive as zeros from the tensor copy and decode to zeros
+                        if (FMT == ALLOYB_Q4_K) decode_q4k<BF16>(row, hdr, g, dst, gate);
+                        else if (FMT == ALLOYB_Q6_K) decode_q6k<BF16>(row + off6, g, dst, gate);
+                        else decode_q8_0<BF16>(stg, g, r, dst, gate);
+                        ok = gate.ok;
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    }
+                    bar_arrive(&bars->full[s]);
+                    // every decode thread releases the super-block once
                     bar_arrive(&bars->p_empty[ps]);
                     if (++ps == static_cast<uint32_t>(pstages)) {
                         ps = 0;
@@ -756,7 +747,6 @@ gemm_tc_kernel(const __grid_constant__ Maps maps, const Params P) {
                 }
             }
         };
-        static_assert(DG == 2 || DG == 4, "groups deal out the four steps of a super-block");
         if (P.format == ALLOYB_Q4_K) decode_all(std::integral_constant<int, ALLOYB_Q4_K>{});
         else if (P.format == ALLOYB_Q6_K) decode_all(std::integral_constant<int, ALLOYB_Q6_K>{});
         else decode_all(std::integral_constant<int, ALLOYB_Q8_0>{});
@@ -953,12 +943,12 @@ static int sm_count_of_device(int& dev) {
 // as many as the SMs, K is split over a cluster per tile: as many ranges as leave all clusters resident at once.  (The
 // partial tiles used to meet in a fixed fp32 scratch by atomic additions, for up to 128 tokens: two such GEMMs on
 // different streams added into each other's sums, and the order of the additions changed from run to run.)
-template <bool BF16, int BM, int DG>
+template <bool BF16, int BM>
 static int launch(const Maps& maps, Params& P, int tiles, int sms, int dev, cudaStream_t st) {
     static bool configured[64] = {};
     static int clusters[64][MAX_SPLITS + 1] = {};
-    using C = Cfg<BM, DG>;
-    auto kern = gemm_tc_kernel<BF16, BM, DG>;
+    using C = Cfg<BM>;
+    auto kern = gemm_tc_kernel<BF16, BM>;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(C::THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
@@ -997,10 +987,10 @@ static int launch(const Maps& maps, Params& P, int tiles, int sms, int dev, cuda
 template <bool BF16>
 static int launch_bm(int BM, const Maps& maps, Params& P, int tiles, int sms, int dev, cudaStream_t st) {
     switch (BM) {
-        case 32: return launch<BF16, 32, 4>(maps, P, tiles, sms, dev, st);
-        case 64: return launch<BF16, 64, 4>(maps, P, tiles, sms, dev, st);
-        case 128: return launch<BF16, 128, 4>(maps, P, tiles, sms, dev, st);
-        default: return launch<BF16, 256, 4>(maps, P, tiles, sms, dev, st);
+        case 32: return launch<BF16, 32>(maps, P, tiles, sms, dev, st);
+        case 64: return launch<BF16, 64>(maps, P, tiles, sms, dev, st);
+        case 128: return launch<BF16, 128>(maps, P, tiles, sms, dev, st);
+        default: return launch<BF16, 256>(maps, P, tiles, sms, dev, st);
     }
 }
 

@@ -305,7 +305,8 @@ extern "C" int alloyb_rope_inplace(void* q, void* k, const int32_t* pos, int pos
     // whole 16-byte pieces of a head's halves: the row kernel, from as many tokens on as its CTAs (one per token) need to fill
     // half the SMs (40 heads of 128: 16 tokens 2.1 us element by element, 2.8 by rows; 64 2.9 / 2.9; 128 3.4 / 3.0; 2048
     // 28.5 / 7.3) and rows that are worth a CTA (10 heads: 96 tokens 2.2 / 2.35, 128 2.3 / 2.3, 400 3.1 / 2.4)
-    if (B >= ROPE_ROWS_MIN_TOKENS && total >= ROPE_ROWS_MIN_PAIRS && dtype != ALLOYB_F32 && D % 16 == 0 && D / 2 <= ROPE_MAX_HALF && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0) {
+    if (B >= ROPE_ROWS_MIN_TOKENS && total >= ROPE_ROWS_MIN_PAIRS && dtype != ALLOYB_F32 && D % 16 == 0 && D / 2 <= ROPE_MAX_HALF &&
+        ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k)) & 15) == 0) {
         const cudaError_t e =
             dtype == ALLOYB_F16
                 ? launch_pdl(rope_rows_kernel<__half>, dim3(B), dim3(256), 0, st, static_cast<__half*>(q), static_cast<__half*>(k), pos, pos_count,

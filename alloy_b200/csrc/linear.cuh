@@ -36,10 +36,11 @@ int try_gemv_stream_mixed(const void* x, int M, int K, int dtype, const WeightSe
                           const void* norm_w, float eps, cudaStream_t stream);
 int gemv_stream_device_error(int clear);
 // A few fp16 tokens (2..SKINNY_MAX_M) against Q4_K / Q6_K matrices (linear_skinny.cu).  Up to 16 tokens it takes Q4_K only,
-// K = 2048 / 4096 / 8192 (the tokens' fragments then live in registers) and more than two tiles per SM: at 16 tokens gate/up
-// 14336 x 4096 takes 29.8 us against 45.5 with the tokens-as-columns kernel, 4096 x 4096 9.9 against 8.5.  From 17 tokens on
-// it takes every shape: 24 tokens 46 against 87 us, 10.8 against 13.0, Q6_K 4096 x 14336 35.5 against 41.6.  From 28 on the
-// tcgen05 GEMM's definition (weights rounded to the activation type) holds.
+// rows of up to 32 super-blocks (16 from nine tokens on; the tokens' fragments then live in registers) and matrices that the
+// tokens-as-columns kernel of linear_mma.cu needs more than one round of CTAs for: the rule and its figures are there.  At 16
+// tokens gate/up 14336 x 4096 takes 29.8 us against 45.5.  From 17 tokens on it takes every shape: 24 tokens 46 against 87 us,
+// 4096 x 4096 10.8 against 13.0, Q6_K 4096 x 14336 35.5 against 41.6.  From 28 on the tcgen05 GEMM's definition (weights
+// rounded to the activation type) holds.
 constexpr int SKINNY_MAX_M = 27;
 int try_linear_skinny(const void* x, int M, int K, int dtype, const WeightSeg* seg, int n_seg, bool gated, int act,
                       const void* residual, cudaStream_t st);
@@ -52,9 +53,9 @@ int try_q8_gemv(const void* x, int M, int K, int dtype, const void* w0, const vo
                 void* y, int N, int64_t ldy, const void* residual, bool gated, int act, bool constant, cudaStream_t st);
 
 // tcgen05 dequant-GEMM for prefill-sized M (one matrix).
-// Fewer tokens go to the GEMV family: the tcgen05 kernel decodes every weight on the CUDA cores at about
-// 2.4e12 weights/s whatever the token count (35 us for 14336 x 4096), and below this the tokens-as-columns
-// GEMV, whose cost grows with the token count, is still ahead.
+// Fewer tokens go to the GEMV family: the tcgen05 kernel takes the same time at any narrow token count (25 us for
+// 14336 x 4096 at 32 and 64 tokens), and below this the kernels of linear_skinny.cu and linear_mma.cu, whose cost grows
+// with the token count, are ahead.
 constexpr int GEMM_TC_MIN_M = 28;
 // `tail`: a second matrix whose packed rows follow seg's in memory, run in the same launch (its rows go to its
 // own output).

@@ -1,5 +1,5 @@
-// Dequant-GEMV / skinny GEMM for a few tokens: fp16 up to 16 (what linear_skinny.cu leaves: Q6_K, matrices of at most two
-// tiles per SM, other K), bf16 up to 27, and the one-token shapes the persistent streaming kernel (linear_stream.cu) does
+// Dequant-GEMV / skinny GEMM for a few tokens: fp16 up to 16 (what linear_skinny.cu leaves: Q6_K, matrices of few row tiles,
+// long rows), bf16 up to 27, and the one-token shapes the persistent streaming kernel (linear_stream.cu) does
 // not take (bf16, K not a multiple of 1024).
 //
 // Why tensor cores on a memory-bound op: at HBM speed a B200 streams ~11.5e12

@@ -13,7 +13,9 @@
 //   may be any weights as long as both operands agree, so the four lanes of a row take different sub-blocks, each lane
 //   needs the scales of its own two only, and reads its weights with 128-bit loads.
 // * The minima (dmin * m * sum of x) are one MMA per super-block: A = the integers m, B = the sums of x per sub-block in two
-//   pieces (22 bits, scaled to fit any activations).  The sums come from MMAs against ones with the TOKENS as rows, whose
+//   pieces (22 bits, scaled to fit any activations).  On tokens whose products cancel, where the output's rounding hides
+//   nothing, the error of the whole sum is 0.07 .. 0.2 x 2^-24 of sum |w x| rms (K = 2048 .. 14336); linear_mma.cu, which
+//   keeps the sums in fp32 and adds up after every 32 weights, leaves 0.4 .. 2.3.  The sums come from MMAs against ones with the TOKENS as rows, whose
 //   accumulator layout is the layout the B operand wants.
 // * Q6_K: codes minus 32 as fp16, one MMA per 16-weight sub-block, the sub-block's d * scale applied in fp32 to the
 //   sums (a product of code and scale would need 12 bits).

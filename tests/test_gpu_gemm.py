@@ -118,9 +118,8 @@ def _weights(fmt, rng, n, k):
 
 
 # Batched-decode and chunk sizes: one token tile of 32 / 64 / 128 columns, ragged token and row
-# counts, matrices with fewer row tiles than SMs (K split over several CTAs whose partial tiles
-# meet in the fp32 scratch), with and without a residual.  Every case runs twice: the second call
-# finds the scratch and the tile counters as the first one left them.
+# counts, matrices with fewer row tiles than SMs (K split over a cluster whose partial tiles meet in
+# distributed shared memory), with and without a residual.
 @pytest.mark.parametrize("fmt,m,n,k,dt", [
     ("q4_k", 28, 4096, 4096, "f16"), ("q4_k", 31, 1024, 4096, "bf16"), ("q4_k", 32, 4096, 14336, "f16"),
     ("q4_k", 64, 14336, 4096, "f16"), ("q4_k", 128, 200, 1024, "bf16"), ("q4_k", 129, 200, 1024, "bf16"),
@@ -153,7 +152,7 @@ def test_gemm_few_tokens_split_k_and_residual(fmt, m, n, k, dt):
 
 
 # Gate/up pairs up to 128 tokens keep two accumulators in tensor memory; few row tiles split K over
-# two planes of the scratch.
+# a cluster, a partial tile of each accumulator.
 @pytest.mark.parametrize("m,n,k,dt", [(32, 14336, 4096, "f16"), (64, 1024, 4096, "bf16"), (128, 3584, 2048, "f16"),
                                       (29, 200, 1024, "f16")])
 @pytest.mark.parametrize("act", ["silu", "gelu"])
