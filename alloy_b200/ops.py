@@ -12,6 +12,11 @@ each op has a ``CUDA`` kernel that calls the C ABI of ``liballoy_b200.so`` on
 the current stream, plus the same ``Meta`` shape functions.  There is no CPU
 implementation, as in the reference: a CPU call raises ``NotImplementedError``.
 
+Calls follow what the stream wrote before them, weights included, with the exception that
+``include/alloy_b200.h`` states for fp16 / bf16 Q4_K and Q6_K linears below 28 tokens: a
+program that rewrites such packed rows on the stream puts one more operation between the
+write and the call.
+
 Two ops have no reference schema: ``attention_cache_q8_paged`` (decode
 attention over the 16-token-paged pool of 34-byte q8_0 blocks) and
 ``linear_residual`` (row-parallel projection with the residual add fused).
