@@ -105,14 +105,19 @@ def test_tokens_in_registers(k):
 
 @pytest.mark.parametrize("fmt,tiles,extra,k", [("q4_k", 6, 131, 512), ("q4_k", 17, 5, 256), ("q6_k", 2, 9, 2048), ("q6_k", 10, 321, 2048)])
 def test_row_groups_and_passes(fmt, tiles, extra, k):
-    """17 tokens and more: two and four row groups, several passes over K, rings that run on from pass to pass."""
+    """17 tokens and more: two and four row groups, several passes over K, rings that run on from pass to pass; dense rows and
+    rows with padding."""
     rng = np.random.default_rng([tiles, k])
     n = _rows(tiles, 16, extra)
     w, deq = _weights(fmt, rng, n, k)
+    op = torch.ops.alloy.gguf_q4_k_mm if fmt == "q4_k" else torch.ops.alloy.gguf_q6_k_mm
+    padded = torch.full((n, w.shape[1] + 48), 0xFF, dtype=torch.uint8, device=DEV)
+    padded[:, :w.shape[1]] = _dev(w)
     for m in (17, 24, 27):
         x = synth.activations(rng, m, k)
-        y = (torch.ops.alloy.gguf_q4_k_mm if fmt == "q4_k" else torch.ops.alloy.gguf_q6_k_mm)(_dev(x), _dev(w))
+        y = op(_dev(x), _dev(w))
         assert_close(to_np(y), _product(x, deq), torch.float16, f"{fmt} {m}x{n}x{k}")
+        assert torch.equal(op(_dev(x), padded[:, :w.shape[1]]), y)
     assert _lib.load().alloyb_device_error(1) == 0
 
 
